@@ -1577,6 +1577,11 @@ void launch_walk(const BHWorkspace &w, unsigned blocks, cudaStream_t st, const u
                                                                          params, P);
 }
 
+// Teams walk cell by cell with two bodies per lane.
+int bh_walk_team(const BHWorkspace &w, int64_t n) {
+    return w.walk == kWalkCell && w.bodies_per_lane == 2 ? bh_team_size(n) : 1;
+}
+
 bool bh_walk_writes_host(const BHWorkspace &w) { return w.walk == kWalkCell && w.bodies_per_lane == 2; }
 
 int bh_walk_form() {
@@ -1590,7 +1595,28 @@ cudaError_t bh_traverse(const float4 *pos_sorted, int64_t n, const BHWorkspace &
     if (host.pos && !bh_walk_writes_host(w)) return cudaErrorInvalidValue;
     if (timer) timer->begin(kStageTraverse, st);
     // The record count P[n] stays on the device; the kernel reads it.
-    if (w.bodies_per_lane == 2) {
+    const int team = bh_walk_team(w, n);
+    if (team > 1) {
+        TeamWalk a;
+        a.nodes = w.nodes;
+        a.kids = w.kids;
+        a.node_total = w.P + n;
+        a.pos = pos_sorted;
+        a.n = n;
+        a.eps2 = eps2;
+        a.theta2 = theta2;
+        a.dt = dt;
+        a.pos_out = pos_out;
+        a.vel = vel;
+        a.acc = acc;
+        a.force_out = force_out;
+        a.ids = ids;
+        a.counters = w.counters;
+        a.euler = euler;
+        a.host = host;
+        const cudaError_t e = bh_team_walk(a, team, !(eps2 > 0.f && theta2 > 0.f), (n + 63) / 64, st);
+        if (e != cudaSuccess) return e;
+    } else if (w.bodies_per_lane == 2) {
         const int64_t warps = (n + 63) / 64;
         const unsigned blocks = static_cast<unsigned>((warps * 32 + 255) / 256);
         if (w.counters)
@@ -1677,16 +1703,41 @@ cudaError_t bh_ensemble_step(int64_t n, BHWorkspace &w, const BHEnsembleTables &
     err = bh_build(Po, n, w, st, status, tm, sv);
     if (err != cudaSuccess) return err;
     if (tm) tm->begin(kStageTraverse, st);
-    const unsigned blocks = static_cast<unsigned>((static_cast<int64_t>(e.nwarps) * 32 + 255) / 256);
-    if (w.counters)
-        launch_walk<true, false, true, true>(w, blocks, st, nullptr, Po, n, 0.f, 0.f, 0.f, P, Vo, Ao, nullptr, nullptr,
-                                             w.counters, nullptr, 0, e.warps, e.nwarps, e.params, w.P);
-    else if (e.all_soft)
-        launch_walk<false, false, true, false>(w, blocks, st, nullptr, Po, n, 0.f, 0.f, 0.f, P, Vo, Ao, nullptr,
-                                               nullptr, nullptr, nullptr, 0, e.warps, e.nwarps, e.params, w.P);
-    else
-        launch_walk<false, false, true, true>(w, blocks, st, nullptr, Po, n, 0.f, 0.f, 0.f, P, Vo, Ao, nullptr, nullptr,
-                                              nullptr, nullptr, 0, e.warps, e.nwarps, e.params, w.P);
+    // One launch per run of systems with the same team size.
+    const int4 *work = e.warps;
+    for (const std::pair<int, int> &run : e.teams) {
+        const int team = w.walk == kWalkCell ? run.first : 1;
+        const int sets = run.second;
+        if (team > 1) {
+            TeamWalk a;
+            a.nodes = w.nodes;
+            a.kids = w.kids;
+            a.pos = Po;
+            a.n = n;
+            a.pos_out = P;
+            a.vel = Vo;
+            a.acc = Ao;
+            a.counters = w.counters;
+            a.work = work;
+            a.params = e.params;
+            a.P = w.P;
+            err = bh_team_walk(a, team, !e.all_soft, sets, st);
+            if (err != cudaSuccess) return err;
+        } else {
+            const unsigned blocks = static_cast<unsigned>((static_cast<int64_t>(sets) * 32 + 255) / 256);
+            if (w.counters)
+                launch_walk<true, false, true, true>(w, blocks, st, nullptr, Po, n, 0.f, 0.f, 0.f, P, Vo, Ao, nullptr,
+                                                     nullptr, w.counters, nullptr, 0, work, sets, e.params, w.P);
+            else if (e.all_soft)
+                launch_walk<false, false, true, false>(w, blocks, st, nullptr, Po, n, 0.f, 0.f, 0.f, P, Vo, Ao,
+                                                       nullptr, nullptr, nullptr, nullptr, 0, work, sets, e.params,
+                                                       w.P);
+            else
+                launch_walk<false, false, true, true>(w, blocks, st, nullptr, Po, n, 0.f, 0.f, 0.f, P, Vo, Ao, nullptr,
+                                                      nullptr, nullptr, nullptr, 0, work, sets, e.params, w.P);
+        }
+        work += sets;
+    }
     if (tm) tm->end(kStageTraverse, st);
     return cudaGetLastError();
 }

@@ -5,6 +5,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <utility>
+#include <vector>
+
 #include "kernels.h"
 
 namespace nbody {
@@ -118,6 +121,30 @@ bool bh_walk_writes_host(const BHWorkspace &w);
 cudaError_t bh_traverse(const float4 *pos_sorted, int64_t n, const BHWorkspace &w, float eps2, float theta2,
                         float dt, float4 *pos_out, float4 *vel, float4 *acc, float4 *force_out, const int *ids,
                         int euler, cudaStream_t st, StageTimer *timer, const HostOut &host = HostOut{});
+// The cell walk by teams of warps (walk_team.cu): `team` warps per set of 64
+// bodies, `sets` sets. work == nullptr: one system of n bodies; else one entry
+// {system, first body of the set, first body and end of the system} per set,
+// with dt, eps2, theta2 and the integrator from params[system] and the records
+// from P. guard: as GUARD of the walks.
+struct TeamWalk {
+    const BHNode *nodes = nullptr;
+    const int *kids = nullptr;
+    const uint32_t *node_total = nullptr;
+    const float4 *pos = nullptr;
+    int64_t n = 0;
+    float eps2 = 0.f, theta2 = 0.f, dt = 0.f;
+    float4 *pos_out = nullptr, *vel = nullptr, *acc = nullptr, *force_out = nullptr;
+    const int *ids = nullptr;
+    unsigned long long *counters = nullptr;
+    int euler = 0;
+    const int4 *work = nullptr;
+    const float4 *params = nullptr;
+    const uint32_t *P = nullptr;
+    HostOut host;
+};
+// Warps per set of a system of n bodies: 1 is cell_walk_kernel.
+int bh_team_size(int64_t n);
+cudaError_t bh_team_walk(const TeamWalk &a, int team, bool guard, int64_t sets, cudaStream_t st);
 // Potential -sum m / sqrt(d^2 + eps^2) of every sorted body over the same
 // accepted records as the forces, into phi_out[ids[b]] (or phi_out[b]).
 cudaError_t bh_potential(const float4 *pos_sorted, int64_t n, const BHWorkspace &w, float eps2, float theta2,
@@ -134,6 +161,8 @@ struct BHEnsembleTables {
     int *fdepth = nullptr;          // per system: the reference's fixed top-level depth
     int4 *warps = nullptr;          // traversal work: system, first body, system first, system end
     int nwarps = 0;
+    // Runs of sets (warps[] entries) whose systems share a team size, in order.
+    std::vector<std::pair<int, int>> teams;  // team size, sets
     float4 *params = nullptr;       // per system: dt, eps2, theta2, euler (0 / 1)
     uint64_t *keys_orig = nullptr;  // per body: unsorted key
     int seg_passes = 1;             // 8-bit digits of the system id

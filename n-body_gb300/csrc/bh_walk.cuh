@@ -1,4 +1,4 @@
-// Device pieces of the Barnes-Hut walks shared by their kernels: the force of a record
+// Device pieces of the Barnes-Hut walks shared by their kernels (bh.cu, walk_team.cu): the force of a record
 // or of a run of bodies, the decision of a record for a set of bodies from its box, the union walk of a subtree,
 // and the fused integrator.
 #pragma once
@@ -22,24 +22,33 @@ __device__ __forceinline__ float float_of(unsigned o) {
 // side A takes part when doA, side B when doB. Per side the arithmetic and
 // its rounding are those of direct_sum_range: a side that does not take part,
 // or a pair it skips (m == 0 or r^2 == 0), adds dx * 0 = +0 to its sums.
+// U bodies are loaded before they are summed (the order of the sums is the
+// same for every U).
+template <int U = 1>
 __device__ __forceinline__ void direct_sum_range2(const float4 *__restrict__ pos, int64_t n, int first, int count,
                                                   float2 nx, float2 ny, float2 nz, float eps2, bool doA, bool doB,
                                                   float2 &ax, float2 &ay, float2 &az) {
     const int q0 = first < 0 ? 0 : first;
     const int q1 = first + count < n ? first + count : static_cast<int>(n);
-    for (int q = q0; q < q1; ++q) {
-        const float4 o = pos[q];
-        const float2 ex = __fadd2_rn(make_float2(o.x, o.x), nx);
-        const float2 ey = __fadd2_rn(make_float2(o.y, o.y), ny);
-        const float2 ez = __fadd2_rn(make_float2(o.z, o.z), nz);
-        const float2 r2 = __fadd2_rn(__fadd2_rn(__fmul2_rn(ex, ex), __fmul2_rn(ey, ey)), __fmul2_rn(ez, ez));
-        const float2 iv = make_float2(rsqrt_ftz(r2.x + eps2), rsqrt_ftz(r2.y + eps2));
-        const float2 w = __fmul2_rn(__fmul2_rn(__fmul2_rn(make_float2(o.w, o.w), iv), iv), iv);
-        const bool ua = doA && o.w > 0.f && r2.x > 0.f, ub = doB && o.w > 0.f && r2.y > 0.f;
-        const float2 ws = make_float2(ua ? w.x : 0.f, ub ? w.y : 0.f);
-        ax = __ffma2_rn(ex, ws, ax);
-        ay = __ffma2_rn(ey, ws, ay);
-        az = __ffma2_rn(ez, ws, az);
+    for (int q = q0; q < q1; q += U) {
+        float4 r[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) r[u] = q + u < q1 ? pos[q + u] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const float4 o = r[u];
+            const float2 ex = __fadd2_rn(make_float2(o.x, o.x), nx);
+            const float2 ey = __fadd2_rn(make_float2(o.y, o.y), ny);
+            const float2 ez = __fadd2_rn(make_float2(o.z, o.z), nz);
+            const float2 r2 = __fadd2_rn(__fadd2_rn(__fmul2_rn(ex, ex), __fmul2_rn(ey, ey)), __fmul2_rn(ez, ez));
+            const float2 iv = make_float2(rsqrt_ftz(r2.x + eps2), rsqrt_ftz(r2.y + eps2));
+            const float2 w = __fmul2_rn(__fmul2_rn(__fmul2_rn(make_float2(o.w, o.w), iv), iv), iv);
+            const bool ua = doA && o.w > 0.f && r2.x > 0.f, ub = doB && o.w > 0.f && r2.y > 0.f;
+            const float2 ws = make_float2(ua ? w.x : 0.f, ub ? w.y : 0.f);
+            ax = __ffma2_rn(ex, ws, ax);
+            ay = __ffma2_rn(ey, ws, ay);
+            az = __ffma2_rn(ez, ws, az);
+        }
     }
 }
 

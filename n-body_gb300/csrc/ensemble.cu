@@ -331,6 +331,7 @@ int relayout(nbody_ensemble *e) {
     if (!bh.empty()) {
         std::vector<int> seg(static_cast<size_t>(bh_n));
         std::vector<int4> chunks, warps;
+        std::vector<std::pair<int, int>> teams;
         std::vector<int> fdepth(bh.size());
         std::vector<float4> prm(bh.size());
         for (size_t g = 0; g < bh.size(); ++g) {
@@ -342,6 +343,9 @@ int relayout(nbody_ensemble *e) {
                 chunks.push_back(make_int4(static_cast<int>(g), f + c * kBBoxChunk,
                                            std::min(end, f + (c + 1) * kBBoxChunk), nch));
             for (int b = f; b < end; b += kWarpBodies) warps.push_back(make_int4(static_cast<int>(g), b, f, end));
+            const int team = nbody::bh_team_size(s.n), sets = static_cast<int>((s.n + kWarpBodies - 1) / kWarpBodies);
+            if (teams.empty() || teams.back().first != team) teams.emplace_back(team, 0);
+            teams.back().second += sets;
             fdepth[g] = nbody::bh_father_depth(s.n);
             prm[g] = make_float4(s.dt, s.eps2, s.theta2, s.euler ? 1.f : 0.f);
         }
@@ -361,6 +365,7 @@ int relayout(nbody_ensemble *e) {
         t.fdepth = take<int>(p, nsys);
         t.warps = take<int4>(p, warps.size());
         t.nwarps = static_cast<int>(warps.size());
+        t.teams = teams;
         t.params = take<float4>(p, nsys);
         t.keys_orig = take<uint64_t>(p, static_cast<size_t>(bh_n));
         t.seg_passes = nsys <= 256 ? 1 : nsys <= 65536 ? 2 : 3;
@@ -781,11 +786,11 @@ int nbody_ensemble_counts(nbody_ensemble *e, int *systems, int64_t *pp_bodies, i
     if (launches_per_step) {
         // direct sum: 1; Barnes-Hut: bbox, keys, histogram + scan + 8 key
         // passes, segment keys + histogram + scan + passes, gather, 7 build
-        // kernels (+ the cell walk's child table), the upsweep's, traversal
+        // kernels (+ the cell walk's child table), the upsweep's, one walk per team size
         int l = e->pp_nitems > 0 ? 1 : 0;
         if (e->bh_n > 0)
             l += 2 + (2 + 8) + (e->tab.systems > 1 ? 3 + e->tab.seg_passes : 0) + 1 + 7 +
-                 (e->ws.walk == nbody::kWalkCell ? 1 : 0) + nbody::bh_upsweep_launches(e->bh_n, true) + 1;
+                 (e->ws.walk == nbody::kWalkCell ? 1 : 0) + nbody::bh_upsweep_launches(e->bh_n, true) + static_cast<int>(e->tab.teams.size());
         *launches_per_step = l;
     }
     return NBODY_OK;

@@ -63,6 +63,7 @@ struct nbody_ctx {
     int *status_host = nullptr;  // page-locked copy of it, read after a stream sync
     void *scratch = nullptr;
     size_t scratch_bytes = 0;
+    size_t scratch_arrivals = 0;  // bytes of arrival counters of the plan that used it last
     bool uploaded = false;
     nbody::EventTimer *timer = nullptr;  // non-null while profiling is enabled
     std::string last_error;
@@ -124,17 +125,37 @@ int fail(nbody_ctx *ctx, cudaError_t e) {
 
 bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-int ensure_scratch(nbody_ctx *ctx, size_t bytes) {
-    if (bytes <= ctx->scratch_bytes) return NBODY_OK;
-    if (ctx->scratch) {
-        NB_CK(ctx, cudaStreamSynchronize(ctx->stream));
-        cudaFree(ctx->scratch);
-        ctx->scratch = nullptr;
-        ctx->scratch_bytes = 0;
+// Scratch for a direct-sum plan of n bodies, its arrival counters zero. Plans
+// of other sizes put partial sums where this one may have its counters, so
+// these are cleared when the plan's layout is not the one used last. A plan
+// that keeps every block's sums apart takes much more scratch than the others:
+// where that cannot be had the plan falls back.
+int ensure_scratch(nbody_ctx *ctx, int64_t n, nbody::PPPlan &plan) {
+    for (;;) {
+        if (plan.partial_bytes <= ctx->scratch_bytes) break;
+        if (ctx->scratch) {
+            NB_CK(ctx, cudaStreamSynchronize(ctx->stream));
+            cudaFree(ctx->scratch);
+            ctx->scratch = nullptr;
+            ctx->scratch_bytes = 0;
+        }
+        const cudaError_t e = cudaMalloc(&ctx->scratch, plan.partial_bytes);
+        if (e == cudaErrorMemoryAllocation && plan.sym.blocks > 0) {
+            cudaGetLastError();
+            ctx->scratch = nullptr;
+            plan = nbody::pp_plan(n, ctx->device, true, false);
+            continue;
+        }
+        NB_CK(ctx, e);
+        NB_CK(ctx, cudaMemsetAsync(ctx->scratch, 0, plan.partial_bytes, ctx->stream));
+        ctx->scratch_bytes = plan.partial_bytes;
+        ctx->scratch_arrivals = plan.arrivals_bytes;
     }
-    NB_CK(ctx, cudaMalloc(&ctx->scratch, bytes));
-    NB_CK(ctx, cudaMemsetAsync(ctx->scratch, 0, bytes, ctx->stream));
-    ctx->scratch_bytes = bytes;
+    if (plan.partial_bytes > 0 && plan.arrivals_bytes != ctx->scratch_arrivals) {
+        if (plan.arrivals_bytes > 0)
+            NB_CK(ctx, cudaMemsetAsync(ctx->scratch, 0, plan.arrivals_bytes, ctx->stream));
+        ctx->scratch_arrivals = plan.arrivals_bytes;
+    }
     return NBODY_OK;
 }
 
@@ -159,8 +180,8 @@ int read_status(nbody_ctx *ctx) {
 }
 
 int pp_steps(nbody_ctx *ctx, int steps) {
-    const nbody::PPPlan plan = nbody::pp_plan(ctx->n, ctx->device);
-    int rc = ensure_scratch(ctx, plan.partial_bytes);
+    nbody::PPPlan plan = nbody::pp_plan(ctx->n, ctx->device);
+    int rc = ensure_scratch(ctx, ctx->n, plan);
     if (rc != NBODY_OK) return rc;
     for (int s = 0; s < steps; ++s) {
         nbody::Integrate g;
@@ -673,8 +694,8 @@ bool pp_update_graphed(nbody_ctx *ctx, const float *positions4, float *velocitie
            *ma = nbody::host_mapped(accelerations4, b4, dev), *mm = nbody::host_mapped(masses4, b4, dev);
     float4 *mf = forces4 ? nbody::host_mapped(forces4, b4, dev) : nullptr;
     if (!(mp && mv && ma && mm && (!forces4 || mf))) return false;
-    const nbody::PPPlan plan = nbody::pp_plan(ctx->n, ctx->device);
-    *rc = ensure_scratch(ctx, plan.partial_bytes);  // allocation stays outside the capture
+    nbody::PPPlan plan = nbody::pp_plan(ctx->n, ctx->device);
+    *rc = ensure_scratch(ctx, ctx->n, plan);  // allocation stays outside the capture
     if (*rc != NBODY_OK) return true;
     auto body = [&]() -> int {
         NB_CK(ctx, nbody::host_gather(mp, mm, mv, ma, ctx->pos[0], ctx->vel, ctx->acc, ctx->n, ctx->stream));
@@ -840,8 +861,8 @@ int nbody_pp_forces_device(nbody_ctx *ctx, const void *pos_mass4, void *force4, 
     if (!ctx || !pos_mass4 || !force4 || n <= 0) return NBODY_ERR_ARG;
     if (!aligned16(pos_mass4) || !aligned16(force4)) return NBODY_ERR_ARG;
     DeviceGuard dg(ctx->device);
-    const nbody::PPPlan plan = nbody::pp_plan(n, ctx->device);
-    int rc = ensure_scratch(ctx, plan.partial_bytes);
+    nbody::PPPlan plan = nbody::pp_plan(n, ctx->device);
+    int rc = ensure_scratch(ctx, n, plan);
     if (rc != NBODY_OK) return rc;
     nbody::Integrate g;
     g.force = static_cast<float4 *>(force4);
@@ -857,8 +878,8 @@ int nbody_pp_step_device(nbody_ctx *ctx, const void *pos_in, void *pos_out, void
         (force4 && !aligned16(force4)))
         return NBODY_ERR_ARG;
     DeviceGuard dg(ctx->device);
-    const nbody::PPPlan plan = nbody::pp_plan(n, ctx->device);
-    int rc = ensure_scratch(ctx, plan.partial_bytes);
+    nbody::PPPlan plan = nbody::pp_plan(n, ctx->device);
+    int rc = ensure_scratch(ctx, n, plan);
     if (rc != NBODY_OK) return rc;
     nbody::Integrate g;
     g.pos_out = static_cast<float4 *>(pos_out);
@@ -878,7 +899,7 @@ int nbody_pp_config(nbody_ctx *ctx, int64_t n, int *bodies_per_thread, int *slic
     const nbody::PPPlan plan = nbody::pp_plan(n, ctx->device);
     if (bodies_per_thread) *bodies_per_thread = plan.k;
     if (slices) *slices = plan.slices;
-    if (ctas) *ctas = plan.linear_ctas > 0 ? plan.linear_ctas : plan.iblocks * plan.slices;
+    if (ctas) *ctas = plan.sym.blocks > 0 ? plan.sym.ctas : plan.linear_ctas > 0 ? plan.linear_ctas : plan.iblocks * plan.slices;
     return NBODY_OK;
 }
 

@@ -38,6 +38,21 @@ struct StageTimer {
     virtual void end(int stage, cudaStream_t s) = 0;
 };
 
+// How the tiles of the direct sum over pairs of blocks (pp_sym.cu) are spread
+// over CTAs; blocks == 0: too many bodies for it.
+constexpr int kSymMaxCtas = 608;
+struct SymPlan {
+    int blocks = 0;     // of 1,024 bodies
+    int window = 0;     // blocks that a block meets in front of it ...
+    int heavy = 0;      // ... and one more for the first `heavy` blocks
+    int row_tiles = 0;  // tiles of a j-row
+    int ctas = 0;
+    int begin[kSymMaxCtas + 1] = {};      // first tile of each CTA's range, and the end
+    size_t parts_bytes = 0, bytes = 0;  // scratch: parts, then j-rows
+};
+SymPlan pp_sym_plan(int64_t n, int sms);
+int pp_sym_bodies_per_thread();
+
 // Launch shape of the direct-sum force kernel for one n.
 struct PPPlan {
     int k = 4;          // i-bodies per thread
@@ -47,9 +62,10 @@ struct PPPlan {
     int linear_ctas = 0;  // > 0: linear split of the (i-block, j-pair) work over this many CTAs
     size_t arrivals_bytes = 0; // per-i-block arrival counters at the start of scratch (zeroed once)
     size_t partial_bytes = 0;  // total scratch: counters + per-slice partial accelerations
+    SymPlan sym;               // sym.blocks > 0: every pair once (pp_sym.cu), partial_bytes as it needs
 };
 
-PPPlan pp_plan(int64_t n, int device, bool allow_linear = true);
+PPPlan pp_plan(int64_t n, int device, bool allow_linear = true, bool allow_sym = true);
 
 // pp_plan with the slice count lowered until the scratch it needs fits in
 // `scratch_bytes` (one slice needs none).
@@ -62,6 +78,9 @@ PPPlan pp_plan_within(int64_t n, int device, size_t scratch_bytes);
 // `status` is a device int.
 cudaError_t pp_launch(const PPPlan &plan, const float4 *pos, int64_t n, float eps2, const Integrate &g,
                       void *scratch, cudaStream_t stream, int *status, StageTimer *timer = nullptr);
+
+cudaError_t pp_sym_launch(const SymPlan &p, const float4 *pos, int64_t n, float eps2, const Integrate &g, void *scratch,
+                          cudaStream_t stream, int *status);
 
 // Packs the reference host layout into the device layout and back.
 cudaError_t pack_state(const float4 *positions4, const float4 *masses4, float4 *pos_mass, int64_t n,

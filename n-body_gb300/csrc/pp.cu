@@ -1,4 +1,5 @@
-// Direct-sum (particle-particle) gravity for sm_103a.
+// Direct-sum (particle-particle) gravity for sm_103a: the launch plans, and the
+// kernels over ordered pairs (pp_sym.cu has the one that takes each pair once).
 //
 // Replaces the reference's PP solvers: the CPU -v 2 force loop
 // (src/ParticleSolver/ParticleSolverCPUParallel/ParticleSolverCPUParallel.cpp:27-40)
@@ -411,13 +412,41 @@ DeviceInfo device_info(int device) {
     return cache[device];
 }
 
+// From here on every pair is evaluated once (GB300, us, ordered / once): 8,192
+// bodies 33 / 35, 9,000 39 / 43, 10,000 45 / 43, 12,000 62 / 55, 16,384 105 / 88,
+// 32,768 388 / 301. Below, a CTA's range is one or two tiles, and its fixed
+// cost and the second kernel outweigh the operations saved.
+constexpr int64_t kSymMinBodies = 10000;
+
+// Every pair once (pp_sym.cu) or every ordered pair: forced by NBODY_PP_SYM = 1
+// / 0; a forced shape of the latter (NBODY_PP_K, _THREADS, _SLICES, _LINEAR)
+// rules the former out.
+bool pp_sym_wanted(int64_t n) {
+    if (std::getenv("NBODY_PP_K") || std::getenv("NBODY_PP_THREADS") || std::getenv("NBODY_PP_SLICES") ||
+        std::getenv("NBODY_PP_LINEAR"))
+        return false;
+    if (const char *e = std::getenv("NBODY_PP_SYM")) return std::atoi(e) == 1;
+    return n >= kSymMinBodies;
+}
+
 int k_index(int k) { return k == 1 ? 0 : k == 2 ? 1 : k == 4 ? 2 : 3; }
 
 }  // namespace
 
-PPPlan pp_plan(int64_t n, int device, bool allow_linear) {
+PPPlan pp_plan(int64_t n, int device, bool allow_linear, bool allow_sym) {
     PPPlan p;
     const DeviceInfo d = device_info(device);
+    if (allow_sym && pp_sym_wanted(n)) {
+        p.sym = pp_sym_plan(n, d.sms > 0 ? d.sms : 1);
+        if (p.sym.blocks > 0) {
+            p.k = pp_sym_bodies_per_thread();
+            p.threads = 256;
+            p.iblocks = p.sym.blocks;
+            p.slices = p.sym.ctas / p.sym.blocks;
+            p.partial_bytes = p.sym.bytes;
+            return p;
+        }
+    }
     // Default shapes from sweeps on GB300 (T x K in {128, 256} x {1, 2, 4, 8},
     // N = 4,096 ... 131,072): from N = 8,192 on, 256 threads with 4 i-bodies
     // each (one CTA per SM at 140 registers, ILP-bound) is fastest; below it 2
@@ -496,7 +525,8 @@ PPPlan pp_plan(int64_t n, int device, bool allow_linear) {
 
 PPPlan pp_plan_within(int64_t n, int device, size_t scratch_bytes) {
     PPPlan p = pp_plan(n, device);
-    if (p.linear_ctas > 0 && p.partial_bytes > scratch_bytes) p = pp_plan(n, device, false);
+    if (p.sym.blocks > 0 && p.partial_bytes > scratch_bytes) p = pp_plan(n, device, true, false);
+    if (p.linear_ctas > 0 && p.partial_bytes > scratch_bytes) p = pp_plan(n, device, false, false);
     while (p.slices > 1 && p.partial_bytes > scratch_bytes) {
         const int64_t fit = static_cast<int64_t>((scratch_bytes > p.arrivals_bytes ? scratch_bytes - p.arrivals_bytes : 0) /
                                                  (static_cast<size_t>(n) * sizeof(float4)));
@@ -538,6 +568,13 @@ static cudaError_t launch_k(const PPPlan &plan, const float4 *pos, int64_t n, fl
 cudaError_t pp_launch(const PPPlan &plan, const float4 *pos, int64_t n, float eps2, const Integrate &g,
                       void *scratch, cudaStream_t stream, int *status, StageTimer *timer) {
     if (n <= 0) return cudaSuccess;
+    if (plan.sym.blocks > 0) {
+        if (!scratch) return cudaErrorInvalidValue;
+        if (timer) timer->begin(kStagePPForce, stream);
+        const cudaError_t e = pp_sym_launch(plan.sym, pos, n, eps2, g, scratch, stream, status);
+        if (timer) timer->end(kStagePPForce, stream);
+        return e;
+    }
     unsigned *arrivals = nullptr;
     float4 *partial = nullptr;
     if (plan.slices > 1 || plan.linear_ctas > 0) {

@@ -17,6 +17,8 @@
 // and writes it out.
 #include <cuda_runtime.h>
 
+#include <cstdlib>
+#include <cstring>
 #include <mutex>
 
 #include "common.cuh"
@@ -33,6 +35,7 @@ constexpr int kSortWarps = kSortThreads / 32;
 constexpr int kItems = 16;  // keys per thread
 constexpr int kTile = kSortThreads * kItems;  // 4096 keys per tile
 constexpr int kPasses = 8;                    // 63 key bits = 8 digits of 8 bits
+constexpr int64_t kMergeSortMax = 1 << 22;  // beyond, merge passes move more than radix passes
 
 constexpr uint32_t kFlagAgg = 1u << 30;   // tile count published
 constexpr uint32_t kFlagIncl = 2u << 30;  // inclusive running total published
@@ -232,6 +235,19 @@ __global__ void __launch_bounds__(kSortThreads, 3)
 
 }  // namespace
 
+bool sort_by_merging(int64_t n) {
+    if (const char *e = std::getenv("NBODY_SORT")) {  // "merge" or "radix" for every size
+        if (std::strcmp(e, "merge") == 0) return true;
+        if (std::strcmp(e, "radix") == 0) return false;
+    }
+    return n <= kMergeSortMax;
+}
+
+int sort_launches(int64_t n, int passes) {
+    if (n <= 1) return 0;
+    return passes == kPasses && sort_by_merging(n) ? merge_sort_launches(n) : 2 + passes;
+}
+
 size_t sort_scratch_bytes(int64_t n) {
     const int64_t tiles = (n + kTile - 1) / kTile;
     size_t b = 0;
@@ -246,8 +262,9 @@ cudaError_t sort_prepare(int device) {
     static bool done[64] = {};
     std::lock_guard<std::mutex> lk(mu);
     if (device >= 0 && device < 64 && done[device]) return cudaSuccess;
-    const cudaError_t e = cudaFuncSetAttribute(onesweep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               static_cast<int>(sizeof(SortSmem)));
+    cudaError_t e = cudaFuncSetAttribute(onesweep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(sizeof(SortSmem)));
+    if (e == cudaSuccess) e = merge_sort_prepare();
     if (e == cudaSuccess && device >= 0 && device < 64) done[device] = true;
     return e;
 }
@@ -261,6 +278,7 @@ cudaError_t sort_pairs(uint64_t *keys, uint32_t *vals, uint64_t *keys_alt, uint3
     cudaError_t e = cudaGetDevice(&device);
     if (e == cudaSuccess) e = sort_prepare(device);
     if (e != cudaSuccess) return e;
+    if (passes == kPasses && sort_by_merging(n)) return merge_sort_pairs(keys, vals, keys_alt, vals_alt, n, stream);
     const int64_t tiles = (n + kTile - 1) / kTile;
     uint32_t *hist = static_cast<uint32_t *>(scratch);
     uint32_t *counters = hist + kPasses * kBins;

@@ -19,4 +19,14 @@ cudaError_t sort_pairs(uint64_t *keys, uint32_t *vals, uint64_t *keys_alt, uint3
                        void *scratch, cudaStream_t stream, int *status, int *result_in_alt, int passes = 8);
 cudaError_t sort_prepare(int device);
 
+// The merge sort (sort_merge.cu) that sort_pairs takes for full keys of up to
+// some size: same result, always left in keys / vals, no scratch.
+bool sort_by_merging(int64_t n);
+// Kernel launches of sort_pairs.
+int sort_launches(int64_t n, int passes = 8);
+int merge_sort_launches(int64_t n);
+cudaError_t merge_sort_prepare();
+cudaError_t merge_sort_pairs(uint64_t *keys, uint32_t *vals, uint64_t *keys_alt, uint32_t *vals_alt, int64_t n,
+                             cudaStream_t stream);
+
 }  // namespace nbody

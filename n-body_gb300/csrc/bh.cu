@@ -398,8 +398,6 @@ __global__ void radix_tree_kernel(const uint64_t *__restrict__ k, int64_t n, Bin
     const int right = (hi == gamma + 1) ? ~static_cast<int>(gamma + 1) : static_cast<int>(gamma + 1);
     t.lo[i] = static_cast<int>(lo);
     t.hi[i] = static_cast<int>(hi);
-    t.left[i] = left;
-    t.right[i] = right;
     t.delta[i] = dnode;
     if (left < 0) t.lparent[~left] = static_cast<int>(i); else t.iparent[left] = static_cast<int>(i);
     if (right < 0) t.lparent[~right] = static_cast<int>(i); else t.iparent[right] = static_cast<int>(i);
@@ -454,19 +452,32 @@ __device__ __forceinline__ int record_of(const BinaryTree &t, const uint32_t *__
 }
 
 // Octree parent of a record: the nearest radix-tree ancestor that is a cell
-// top (the nodes in between split the same cell; at most 6 of them).
-__device__ __forceinline__ int octree_parent(const BinaryTree &t, const uint32_t *__restrict__ mask,
-                                             const uint32_t *__restrict__ P, int p, int base) {
+// top (the nodes in between split the same cell; at most 6 of them), or -1.
+__device__ __forceinline__ int parent_top(const BinaryTree &t, int p) {
     // At most 6 nodes per octree level inside a system, and at most 32 joining
     // nodes (strictly decreasing delta < 32) above a system's subtree.
     for (int guard = 0; p >= 0 && !t.top[p] && guard < 160; ++guard) p = t.iparent[p];
-    return (p >= 0 && t.top[p]) ? record_of(t, mask, P, p, base) : -1;
+    return p >= 0 && t.top[p] ? p : -1;
+}
+
+// Record idx, whose bodies' first key is `key`, into its parent's row of the
+// child table (8 places per cell, by key digit, -1 before). p: its radix-tree
+// parent. Returns the parent record (-1: a root).
+__device__ __forceinline__ int link_child(const BinaryTree &t, const uint32_t *__restrict__ mask,
+                                          const uint32_t *__restrict__ P, int p, int base, uint64_t key, int idx,
+                                          int *__restrict__ kids) {
+    p = parent_top(t, p);
+    if (p < 0) return -1;
+    const int par = record_of(t, mask, P, p, base);
+    const int digit = static_cast<int>(key >> (63 - 3 * (level_c(t.delta[p], base) + 1))) & 7;
+    kids[8 * static_cast<int64_t>(par) + digit] = idx;
+    return par;
 }
 
 __global__ void emit_cells_kernel(const uint64_t *__restrict__ k, int64_t n, BinaryTree t,
                                   const uint32_t *__restrict__ mask, const uint32_t *__restrict__ P,
-                                  const float *__restrict__ box, BHNode *__restrict__ nodes, Records r, SegView sv,
-                                  bool parents) {
+                                  const float *__restrict__ box, BHNode *__restrict__ nodes, Records r,
+                                  int *__restrict__ kids, SegView sv, bool parents) {
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n - 1) return;
     if (!t.top[i]) return;
@@ -483,16 +494,14 @@ __global__ void emit_cells_kernel(const uint64_t *__restrict__ k, int64_t n, Bin
     }
     nodes[idx].meta = meta;
     r.level[idx] = L;
-    if (parents) {  // the climbing upsweep's links
-        const int par = i == 0 ? -1 : octree_parent(t, mask, P, t.iparent[i], base);
-        r.parent[idx] = par;
-        if (par >= 0) atomicAdd(&r.nchild[par], 1);
-    }
+    const int par = i == 0 ? -1 : link_child(t, mask, P, t.iparent[i], base, k[lo], idx, kids);
+    if (parents) r.parent[idx] = par;  // for the climbing upsweep
 }
 
 __global__ void emit_leaves_kernel(const uint64_t *__restrict__ k, int64_t n, const float4 *__restrict__ pos,
                                    BinaryTree t, const uint32_t *__restrict__ mask, const uint32_t *__restrict__ P,
-                                   BHNode *__restrict__ nodes, Records r, SegView sv, bool parents) {
+                                   BHNode *__restrict__ nodes, Records r, int *__restrict__ kids, SegView sv,
+                                   bool parents) {
     const int64_t b = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (b >= n) return;
     const bool lone = !((b > 0 && same_key(k, sv, b, b - 1)) || (b + 1 < n && same_key(k, sv, b, b + 1)));
@@ -501,48 +510,15 @@ __global__ void emit_leaves_kernel(const uint64_t *__restrict__ k, int64_t n, co
     nodes[idx].cm = pos[b];
     nodes[idx].meta = make_int4(__float_as_int(-1.f), static_cast<int>(P[b + 1]), static_cast<int>(b), 1);
     r.level[idx] = kMaxLevel + 1;  // a lone body
-    if (parents) {
-        const int par = n < 2 ? -1 : octree_parent(t, mask, P, t.lparent[b], sv.seg ? 32 : 0);
-        r.parent[idx] = par;
-        if (par >= 0) atomicAdd(&r.nchild[par], 1);
-    }
+    const int par = n < 2 ? -1 : link_child(t, mask, P, t.lparent[b], sv.seg ? 32 : 0, k[b], idx, kids);
+    if (parents) r.parent[idx] = par;
 }
 
-// kids[8 r + j]: the record of the j-th child of cell r in pre-order (the
-// chain r + 1, next(r + 1), ... before next(r)), -1 after the last; a cell
-// has at most 8. Leaves and buckets get no entry. For the cell walk, which
-// decides a cell's children side by side.
-__global__ void kids_kernel(const BHNode *__restrict__ nodes, const uint32_t *__restrict__ total, int64_t cap,
-                            int *__restrict__ kids, int *status) {
-    const int64_t r = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const int64_t m = static_cast<int64_t>(*total) < cap ? static_cast<int64_t>(*total) : cap;
-    if (r >= m) return;
-    const int4 meta = nodes[r].meta;
-    if (__int_as_float(meta.x) < 0.f) return;  // a leaf or a bucket
-    const int64_t end = meta.y < m ? meta.y : m;
-    int k[8];
-    int64_t c = r + 1;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        k[j] = -1;
-        if (c < end) {
-            k[j] = static_cast<int>(c);
-            const int64_t nx = nodes[c].meta.y;
-            c = nx > c ? nx : end;
-        }
-    }
-    if (c < end) record_error(status, NBODY_ERR_CAPACITY);  // more than 8 children: broken tree
-    int4 *out = reinterpret_cast<int4 *>(kids + 8 * r);
-    out[0] = make_int4(k[0], k[1], k[2], k[3]);
-    out[1] = make_int4(k[4], k[5], k[6], k[7]);
-}
-
-// The reference's child order (Octree::getNextNode, src/Octree/Octree.cpp:148-153):
-// index bit a is set when the body lies below the centre on axis a (x = bit 0),
-// while a Morton digit bit is set for the upper half (x = bit 2).
-__device__ __forceinline__ int reference_child_index(uint32_t digit) {
-    return static_cast<int>(((~digit >> 2) & 1u) | ((~digit) & 2u) | (((~digit) & 1u) << 2));
-}
+// The key digit of the child with index q in the reference's order
+// (Octree::getNextNode, src/Octree/Octree.cpp:148-153): bit a of the index is set when
+// the body lies below the centre on axis a (x = bit 0), a digit's bit for the
+// upper half (x = bit 2).
+__device__ constexpr int digit_of_child(int q) { return ((~q & 1) << 2) | (~q & 2) | ((~q >> 2) & 1); }
 
 // Bottom-up centres of mass in the reference's arithmetic
 // (ParallelOctreeCPU::propagate / Octree::propagate, Octree.cpp:238-258): a
@@ -557,37 +533,6 @@ __device__ __forceinline__ int reference_child_index(uint32_t digit) {
 // arrive at a cell computes it and climbs on) and the level schedule (bucket
 // leaves, then one launch per octree level from the deepest up, no atomics),
 // which is faster from about 2^21 bodies and for ensembles.
-// A cell's children by the reference's child index, in registers: each store
-// is eight predicated selects, so no slot is addressed dynamically. The level
-// schedule uses it (0.375 vs 0.481 ms at 4M bodies against an array in local
-// memory, whose traffic reached DRAM); the climb keeps the local array, which
-// costs it fewer registers and so more threads in flight (0.189 vs 0.258 ms
-// at 2^20).
-struct ChildSlots {
-    float4 s[8];
-    unsigned used = 0;
-    __device__ __forceinline__ void put(int j, float4 v) {
-#pragma unroll
-        for (int q = 0; q < 8; ++q) s[q] = j == q ? v : s[q];
-        used |= 1u << j;
-    }
-    // Sum(c * m) / Sum(m) over the occupied slots in index order, every step
-    // rounded on its own.
-    __device__ __forceinline__ float4 centre() const {
-        float cx = 0.f, cy = 0.f, cz = 0.f, m = 0.f;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            if (!((used >> j) & 1u)) continue;
-            cx = __fadd_rn(cx, __fmul_rn(s[j].x, s[j].w));
-            cy = __fadd_rn(cy, __fmul_rn(s[j].y, s[j].w));
-            cz = __fadd_rn(cz, __fmul_rn(s[j].z, s[j].w));
-            m = __fadd_rn(m, s[j].w);
-        }
-        return m > 0.f ? make_float4(__fdiv_rn(cx, m), __fdiv_rn(cy, m), __fdiv_rn(cz, m), m)
-                       : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-};
-
 __device__ __forceinline__ float4 round_trips(float4 c, int times) {
     for (int q = 0; q < times; ++q) {
         c.x = __fdiv_rn(__fmul_rn(c.x, c.w), c.w);
@@ -595,6 +540,66 @@ __device__ __forceinline__ float4 round_trips(float4 c, int times) {
         c.z = __fdiv_rn(__fmul_rn(c.z, c.w), c.w);
     }
     return c;
+}
+
+// The children of a cell, by key digit (-1: none).
+struct KidRow {
+    int c[8];
+    __device__ __forceinline__ KidRow(const int *__restrict__ kids, int rec) {
+        const int4 *row = reinterpret_cast<const int4 *>(kids + 8 * static_cast<int64_t>(rec));
+        const int4 a = row[0], b = row[1];
+        c[0] = a.x, c[1] = a.y, c[2] = a.z, c[3] = a.w;
+        c[4] = b.x, c[5] = b.y, c[6] = b.z, c[7] = b.w;
+    }
+    __device__ __forceinline__ unsigned count() const {
+        unsigned k = 0;
+#pragma unroll
+        for (int d = 0; d < 8; ++d) k += c[d] >= 0 ? 1u : 0u;
+        return k;
+    }
+};
+
+// Centre of mass of a level-L cell from its children: sum(c * m) / sum(m) over
+// the occupied ones in the reference's order, every step rounded on its own.
+// Their loads are in flight together (along the chain of `next` links each
+// waited for the one before: GB300, climb of 4,096 bodies 55 against 25 us,
+// 65,536 68 against 31, 2^20 185 against 160). *bodies: their bodies if all are leaves, else 0.
+__device__ __forceinline__ float4 cell_cm(const BHNode *nodes, const int *__restrict__ level, const KidRow &row, int L,
+                                          int father_depth, int *bodies) {
+    float4 cm[8];
+    int lv[8], w[8];
+#pragma unroll
+    for (int d = 0; d < 8; ++d) {
+        const bool in = row.c[d] >= 0;
+        cm[d] = in ? __ldcg(&nodes[row.c[d]].cm) : make_float4(0.f, 0.f, 0.f, 0.f);
+        w[d] = in ? __ldcg(&nodes[row.c[d]].meta.w) : 0;
+        lv[d] = in ? level[row.c[d]] : 0;
+    }
+    float cx = 0.f, cy = 0.f, cz = 0.f, m = 0.f;
+    int sum = 0;
+    bool leaves = true;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const int d = digit_of_child(q);
+        if (row.c[d] < 0) continue;
+        int trips;
+        if (lv[d] >= kMaxLevel) {  // a leaf (lone body or bucket)
+            trips = father_depth - (L + 1) > 0 ? father_depth - (L + 1) : 0;
+            sum += w[d];
+        } else {
+            trips = lv[d] - L - 1;
+            leaves = false;
+        }
+        if (!(cm[d].w > 0.f)) continue;
+        const float4 o = round_trips(cm[d], trips);
+        cx = __fadd_rn(cx, __fmul_rn(o.x, o.w));
+        cy = __fadd_rn(cy, __fmul_rn(o.y, o.w));
+        cz = __fadd_rn(cz, __fmul_rn(o.z, o.w));
+        m = __fadd_rn(m, o.w);
+    }
+    *bodies = leaves ? sum : 0;
+    return m > 0.f ? make_float4(__fdiv_rn(cx, m), __fdiv_rn(cy, m), __fdiv_rn(cz, m), m)
+                   : make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
 // Centre of mass of the bucket (bodies with identical keys) whose first body
@@ -616,8 +621,8 @@ __device__ __forceinline__ float4 bucket_cm(const uint64_t *__restrict__ k, int6
 
 __global__ void upsweep_climb_kernel(const uint64_t *__restrict__ k, int64_t n, const float4 *__restrict__ pos,
                                      const uint32_t *__restrict__ mask, const uint32_t *__restrict__ P,
-                                     BHNode *__restrict__ nodes, Records r, int father_depth, int *status,
-                                     SegView sv) {
+                                     BHNode *nodes, Records r, const int *__restrict__ kids, int father_depth,
+                                     int *status, SegView sv) {
     const int64_t b = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (b >= n) return;
     if (sv.seg) father_depth = sv.fdepth[sv.seg[b]];
@@ -633,54 +638,18 @@ __global__ void upsweep_climb_kernel(const uint64_t *__restrict__ k, int64_t n, 
     } else {
         return;
     }
+    int par = r.parent[rec];
     for (int depth = 0; depth <= kMaxLevel + 2; ++depth) {
-        const int par = r.parent[rec];
         if (par < 0) return;
         __threadfence();
-        const int done = static_cast<int>(atomicAdd(&r.arrive[par], 1u)) + 1;
-        if (done < __ldcg(&r.nchild[par])) return;
+        const KidRow row(kids, par);
+        const int L = r.level[par], next = r.parent[par];
+        if (atomicAdd(&r.arrive[par], 1u) + 1u < row.count()) return;
         __threadfence();
-        const int L = __ldcg(&r.level[par]);
-        const int4 pm = __ldcg(&nodes[par].meta);
-        float4 slot[8];
-        bool used[8] = {false, false, false, false, false, false, false, false};
-        bool all_leaves = true;
-        int bodies = 0;
-        int c = par + 1;
-        for (int guard = 0; c < pm.y && guard < 8; ++guard) {
-            const int4 cmeta = __ldcg(&nodes[c].meta);
-            float4 cc = __ldcg(&nodes[c].cm);
-            const int cl = __ldcg(&r.level[c]);
-            const uint32_t digit = static_cast<uint32_t>(k[cmeta.z] >> (63 - 3 * (L + 1))) & 7u;
-            int trips;
-            if (cl > kMaxLevel || cl == kMaxLevel) {  // a leaf (lone body or bucket)
-                trips = father_depth - (L + 1) > 0 ? father_depth - (L + 1) : 0;
-                bodies += cmeta.w;
-            } else {
-                trips = cl - L - 1;
-                all_leaves = false;
-            }
-            if (cc.w > 0.f) {
-                const int j = reference_child_index(digit);
-                slot[j] = round_trips(cc, trips);
-                used[j] = true;
-            }
-            c = cmeta.y;
-        }
-        if (c != pm.y) record_error(status, NBODY_ERR_CAPACITY);  // more than 8 children: broken tree
-        float cx = 0.f, cy = 0.f, cz = 0.f, m = 0.f;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            if (!used[j]) continue;
-            cx = __fadd_rn(cx, __fmul_rn(slot[j].x, slot[j].w));
-            cy = __fadd_rn(cy, __fmul_rn(slot[j].y, slot[j].w));
-            cz = __fadd_rn(cz, __fmul_rn(slot[j].z, slot[j].w));
-            m = __fadd_rn(m, slot[j].w);
-        }
-        nodes[par].cm = m > 0.f ? make_float4(__fdiv_rn(cx, m), __fdiv_rn(cy, m), __fdiv_rn(cz, m), m)
-                                : make_float4(0.f, 0.f, 0.f, 0.f);
-        if (all_leaves) nodes[par].meta.w = -bodies;
-        rec = par;
+        int bodies;
+        nodes[par].cm = cell_cm(nodes, r.level, row, L, father_depth, &bodies);
+        if (bodies > 0) nodes[par].meta.w = -bodies;
+        par = next;
     }
     record_error(status, NBODY_ERR_CAPACITY);  // deeper than any octree: broken tree
 }
@@ -752,40 +721,18 @@ __global__ void level_scatter_kernel(const int *__restrict__ level, const uint32
 
 // The cells of one level: each sums its children (already final) in the
 // reference's child order.
-// Four CTAs per SM (64 registers): the eight register slots fit without spills.
 __global__ void __launch_bounds__(256, 4)
-    level_cm_kernel(int L, const uint64_t *__restrict__ k, int64_t n, BHNode *__restrict__ nodes,
-                    const int *__restrict__ level, const unsigned *__restrict__ list, const unsigned *__restrict__ lvl,
-                    int father_depth, int *status, SegView sv) {
+    level_cm_kernel(int L, BHNode *nodes, const int *__restrict__ level, const int *__restrict__ kids,
+                    const unsigned *__restrict__ list, const unsigned *__restrict__ lvl,
+                    int father_depth, SegView sv) {
     const unsigned count = lvl[L], first = lvl[32 + L];
     const unsigned stride = gridDim.x * blockDim.x;
     for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += stride) {
         const int par = static_cast<int>(list[first + q]);
-        const int4 pm = nodes[par].meta;
-        const int fd = sv.seg ? sv.fdepth[sv.seg[pm.z]] : father_depth;
-        ChildSlots slot;
-        bool all_leaves = true;
-        int bodies = 0;
-        int c = par + 1;
-        for (int guard = 0; c < pm.y && guard < 8; ++guard) {
-            const int4 cmeta = nodes[c].meta;
-            const float4 cc = nodes[c].cm;
-            const int cl = level[c];
-            const uint32_t digit = static_cast<uint32_t>(k[cmeta.z] >> (63 - 3 * (L + 1))) & 7u;
-            int trips;
-            if (cl >= kMaxLevel) {  // a leaf (lone body or bucket)
-                trips = fd - (L + 1) > 0 ? fd - (L + 1) : 0;
-                bodies += cmeta.w;
-            } else {
-                trips = cl - L - 1;
-                all_leaves = false;
-            }
-            if (cc.w > 0.f) slot.put(reference_child_index(digit), round_trips(cc, trips));
-            c = cmeta.y;
-        }
-        if (c != pm.y) record_error(status, NBODY_ERR_CAPACITY);  // more than 8 children: broken tree
-        nodes[par].cm = slot.centre();
-        if (all_leaves) nodes[par].meta.w = -bodies;
+        const int fd = sv.seg ? sv.fdepth[sv.seg[nodes[par].meta.z]] : father_depth;
+        int bodies;
+        nodes[par].cm = cell_cm(nodes, level, KidRow(kids, par), L, fd, &bodies);
+        if (bodies > 0) nodes[par].meta.w = -bodies;
     }
 }
 
@@ -1415,15 +1362,12 @@ size_t bh_workspace_layout(int64_t n, void *base, BHWorkspace *w) {
     w->bbox_counter = static_cast<unsigned *>(take(sizeof(unsigned) * 4));
     w->tree.lo = static_cast<int *>(take(sizeof(int) * nn));
     w->tree.hi = static_cast<int *>(take(sizeof(int) * nn));
-    w->tree.left = static_cast<int *>(take(sizeof(int) * nn));
-    w->tree.right = static_cast<int *>(take(sizeof(int) * nn));
     w->tree.delta = static_cast<int *>(take(sizeof(int) * nn));
     w->tree.iparent = static_cast<int *>(take(sizeof(int) * nn));
     w->tree.lparent = static_cast<int *>(take(sizeof(int) * nn));
     w->tree.top = static_cast<int *>(take(sizeof(int) * nn));
     w->rec.level = static_cast<int *>(take(sizeof(int) * 2 * nn));
     w->rec.parent = static_cast<int *>(take(sizeof(int) * 2 * nn));
-    w->rec.nchild = static_cast<int *>(take(sizeof(int) * 2 * nn));
     w->rec.arrive = static_cast<unsigned *>(take(sizeof(unsigned) * 2 * nn));
     w->rec.list = w->rec.arrive;  // one schedule or the other per build
     w->rec.lvl = static_cast<unsigned *>(take(sizeof(unsigned) * 96));
@@ -1513,25 +1457,20 @@ cudaError_t bh_build(const float4 *pos_sorted, int64_t n, BHWorkspace &w, cudaSt
     const bool levels = bh_upsweep_by_levels(n, sv.seg != nullptr);
     // Records: at most 2n (n - 1 cells and n leaves).
     const int64_t cap = 2 * (n > 1 ? n : 2);
-    if (!levels) {
-        e = cudaMemsetAsync(w.rec.nchild, 0, sizeof(int) * static_cast<size_t>(cap), st);
-        if (e == cudaSuccess) e = cudaMemsetAsync(w.rec.arrive, 0, sizeof(unsigned) * static_cast<size_t>(cap), st);
-        if (e != cudaSuccess) return e;
-    }
+    e = cudaMemsetAsync(w.kids, 0xff, sizeof(int) * 8 * static_cast<size_t>(cap), st);
+    if (e == cudaSuccess && !levels)
+        e = cudaMemsetAsync(w.rec.arrive, 0, sizeof(unsigned) * static_cast<size_t>(cap), st);
+    if (e != cudaSuccess) return e;
     if (n >= 2)
         emit_cells_kernel<<<grid_for(n - 1, 256), 256, 0, st>>>(k, n, w.tree, w.mask, w.P, w.box, w.nodes, w.rec,
-                                                                sv, !levels);
-    emit_leaves_kernel<<<grid_for(n, 256), 256, 0, st>>>(k, n, pos_sorted, w.tree, w.mask, w.P, w.nodes, w.rec, sv,
-                                                         !levels);
-    if (w.walk == kWalkCell) {
-        const int64_t cap = 2 * (n > 1 ? n : 2);
-        kids_kernel<<<grid_for(cap, 256), 256, 0, st>>>(w.nodes, w.P + n, cap, w.kids, status);
-    }
+                                                                w.kids, sv, !levels);
+    emit_leaves_kernel<<<grid_for(n, 256), 256, 0, st>>>(k, n, pos_sorted, w.tree, w.mask, w.P, w.nodes, w.rec,
+                                                         w.kids, sv, !levels);
     if (timer) timer->end(kStageBuild, st);
     if (timer) timer->begin(kStageUpsweep, st);
     if (!levels) {
         upsweep_climb_kernel<<<grid_for(n, 256), 256, 0, st>>>(k, n, pos_sorted, w.mask, w.P, w.nodes, w.rec,
-                                                               father_depth(n), status, sv);
+                                                               w.kids, father_depth(n), status, sv);
         if (timer) timer->end(kStageUpsweep, st);
         return cudaGetLastError();
     }
@@ -1544,7 +1483,8 @@ cudaError_t bh_build(const float4 *pos_sorted, int64_t n, BHWorkspace &w, cudaSt
                                                              status);
     const int fd = father_depth(n);
     for (int L = kMaxLevel - 1; L >= 0; --L)
-        level_cm_kernel<<<spread, 256, 0, st>>>(L, k, n, w.nodes, w.rec.level, w.rec.list, w.rec.lvl, fd, status, sv);
+        level_cm_kernel<<<spread, 256, 0, st>>>(L, w.nodes, w.rec.level, w.kids, w.rec.list, w.rec.lvl, fd,
+                                                sv);
     if (timer) timer->end(kStageUpsweep, st);
     return cudaGetLastError();
 }
@@ -1566,8 +1506,8 @@ void launch_walk(const BHWorkspace &w, unsigned blocks, cudaStream_t st, const u
         }
     }
     if (w.walk == kWalkCell)
-        cell_walk_kernel<COUNT, POT, SEG, GUARD><<<blocks * 4, 64, 0, st>>>(w.nodes, w.kids, node_total, pos, n, eps2,
-                                                                         theta2, dt, pos_out, vel, acc, force_out,
+        cell_walk_kernel<COUNT, POT, SEG, GUARD><<<blocks * 4, 64, 0, st>>>(w.nodes, w.kids, node_total,
+                                                                         pos, n, eps2, theta2, dt, pos_out, vel, acc, force_out,
                                                                          ids, counters, phi_out, euler, work, nwork,
                                                                          params, P, host);
     else

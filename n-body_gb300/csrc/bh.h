@@ -25,19 +25,19 @@ struct __align__(16) BHNode {
 };
 
 // Binary radix tree over sorted keys: internal node i covers bodies
-// [lo, hi]; a child < 0 is body ~child.
+// [lo, hi].
 struct BinaryTree {
-    int *lo, *hi, *left, *right, *delta, *iparent, *lparent, *top;
+    int *lo, *hi, *delta, *iparent, *lparent, *top;
 };
 
 // Per-record bookkeeping for the bottom-up pass: level[r] = octree level of
 // record r (kMaxLevel for a bucket, kMaxLevel + 1 for a lone body). The
-// climbing schedule uses parent (octree parent record), nchild and arrive;
+// climbing schedule uses parent (octree parent record) and arrive;
 // the level schedule uses list (the cell records grouped by level; it shares
 // arrive's storage) and lvl: lvl[0..32) = cells per level, lvl[32..64) = where
 // each level's group starts in list, lvl[64..96) = fill cursors.
 struct Records {
-    int *level, *parent, *nchild;
+    int *level, *parent;
     unsigned *arrive;
     unsigned *list;
     unsigned *lvl;
@@ -72,7 +72,7 @@ struct BHWorkspace {
     uint32_t *P = nullptr;  // n + 1 entries; P[n] = record count
     uint32_t *scan_sums = nullptr;
     BHNode *nodes = nullptr;  // up to 2n records
-    int *kids = nullptr;      // 8 child records per cell record (cell walk)
+    int *kids = nullptr;      // child table: 8 places per cell record, by key digit; -1: no child
     // Traversal counters (pairwise evaluations, warp record visits): the
     // traversal counts into `counters` when it is set (= counter_mem).
     unsigned long long *counter_mem = nullptr;

@@ -459,12 +459,12 @@ def bench_bh(args, world, rank, local, dist):
            "d2h_bytes_per_step": 4 * 16 * n, "ms_per_step": round(e2e_s * 1e3 / e2e_steps, 3), "steps": e2e_steps,
            "api": "nbody_update_host (ParticleSolver::updateParticlePositions)"}
     # bbox, keys, sort (a launch over tiles and one per merge pass up to 2^22
-    # bodies, else histogram, scan, 8 passes), gather, 7 build kernels,
+    # bodies, else histogram, scan, 8 passes), gather, 3 build kernels,
     # the upsweep (one climbing launch below 2^21 bodies; from there bucket
     # centres, level count, level scatter and one launch per octree level: 24), walk
     tiles = -(-n // (2048 if n <= 1 << 18 else 4096))
     sort_launches = 10 if n > 1 << 22 else 1 + (tiles - 1).bit_length()
-    launches_per_step = 11 + sort_launches + (1 if n < (1 << 21) else 24)
+    launches_per_step = 7 + sort_launches + (1 if n < (1 << 21) else 24)
     line = {"metric": METRIC, "component": "BH body-steps/s", "value": value, "unit": "body-steps/s",
             "n_gpus": world, "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms / args.steps,
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32", "data": "synthetic",

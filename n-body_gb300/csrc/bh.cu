@@ -79,8 +79,33 @@ __device__ __forceinline__ const float *box_of(const SegView &sv, const float *b
 // ------------------------------------------------------------- bounding box
 // Reference seeds: min = FLT_MAX, max = FLT_MIN (ParallelOctreeCPU.cpp:77-82),
 // strict comparisons. min/max are order-independent, so the result is exact.
+// The block's box from every thread's, in all threads of warp 0; a strict
+// comparison passes over a NaN, and so do the warp reductions.
+__device__ __forceinline__ void block_box(float (&mn)[3], float (&mx)[3], float (*wm)[6]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        mn[a] = warp_min(mn[a]);
+        mx[a] = warp_max(mx[a]);
+        if (lane == 0) {
+            wm[warp][a] = mn[a];
+            wm[warp][3 + a] = mx[a];
+        }
+    }
+    __syncthreads();
+    if (warp == 0) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            mn[a] = warp_min(lane < nw ? wm[lane][a] : FLT_MAX);
+            mx[a] = warp_max(lane < nw ? wm[lane][3 + a] : FLT_MIN);
+        }
+    }
+}
+
 __global__ void bbox_kernel(const float4 *__restrict__ pos, int64_t n, float *__restrict__ partial,
                             unsigned *__restrict__ counter, float *__restrict__ box) {
+    __shared__ float wm[32][6];
+    __shared__ bool last;
     float mn[3] = {FLT_MAX, FLT_MAX, FLT_MAX};
     float mx[3] = {FLT_MIN, FLT_MIN, FLT_MIN};
     const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
@@ -93,33 +118,13 @@ __global__ void bbox_kernel(const float4 *__restrict__ pos, int64_t n, float *__
         if (p.y > mx[1]) mx[1] = p.y;
         if (p.z > mx[2]) mx[2] = p.z;
     }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            const float o1 = __shfl_down_sync(0xffffffffu, mn[a], off);
-            const float o2 = __shfl_down_sync(0xffffffffu, mx[a], off);
-            if (o1 < mn[a]) mn[a] = o1;
-            if (o2 > mx[a]) mx[a] = o2;
-        }
-    }
-    __shared__ float wm[32][6];
-    __shared__ bool last;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    if (lane == 0) {
-        for (int a = 0; a < 3; ++a) {
-            wm[warp][a] = mn[a];
-            wm[warp][3 + a] = mx[a];
-        }
-    }
-    __syncthreads();
+    block_box(mn, mx, wm);
     if (threadIdx.x == 0) {
-        for (int w = 1; w < nw; ++w)
-            for (int a = 0; a < 3; ++a) {
-                if (wm[w][a] < wm[0][a]) wm[0][a] = wm[w][a];
-                if (wm[w][3 + a] > wm[0][3 + a]) wm[0][3 + a] = wm[w][3 + a];
-            }
-        for (int a = 0; a < 6; ++a) partial[blockIdx.x * 6 + a] = wm[0][a];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            partial[blockIdx.x * 6 + a] = mn[a];
+            partial[blockIdx.x * 6 + 3 + a] = mx[a];
+        }
         __threadfence();
         last = atomicAdd(counter, 1u) == gridDim.x - 1;
     }
@@ -128,35 +133,26 @@ __global__ void bbox_kernel(const float4 *__restrict__ pos, int64_t n, float *__
     // Last block: every thread folds a strided share of the partials, then
     // the block reduces as above.
     __threadfence();
-    float r[6] = {FLT_MAX, FLT_MAX, FLT_MAX, FLT_MIN, FLT_MIN, FLT_MIN};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        mn[a] = FLT_MAX;
+        mx[a] = FLT_MIN;
+    }
     for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x)
+#pragma unroll
         for (int a = 0; a < 3; ++a) {
             const float lo = __ldcg(&partial[b * 6 + a]);
             const float hi = __ldcg(&partial[b * 6 + 3 + a]);
-            if (lo < r[a]) r[a] = lo;
-            if (hi > r[3 + a]) r[3 + a] = hi;
+            if (lo < mn[a]) mn[a] = lo;
+            if (hi > mx[a]) mx[a] = hi;
         }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
+    block_box(mn, mx, wm);
+    if (threadIdx.x == 0) {
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            const float o1 = __shfl_down_sync(0xffffffffu, r[a], off);
-            const float o2 = __shfl_down_sync(0xffffffffu, r[3 + a], off);
-            if (o1 < r[a]) r[a] = o1;
-            if (o2 > r[3 + a]) r[3 + a] = o2;
+            box[a] = mn[a];
+            box[3 + a] = mx[a];
         }
-    }
-    __syncthreads();
-    if (lane == 0)
-        for (int a = 0; a < 6; ++a) wm[warp][a] = r[a];
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < nw; ++w)
-            for (int a = 0; a < 3; ++a) {
-                if (wm[w][a] < wm[0][a]) wm[0][a] = wm[w][a];
-                if (wm[w][3 + a] > wm[0][3 + a]) wm[0][3 + a] = wm[w][3 + a];
-            }
-        for (int a = 0; a < 6; ++a) box[a] = wm[0][a];
         *counter = 0u;
     }
 }
@@ -341,9 +337,10 @@ __global__ void gather_kernel(const uint32_t *__restrict__ perm, int64_t n, cons
                               const int *__restrict__ id_in, float4 *__restrict__ pos_out,
                               float4 *__restrict__ vel_out, float4 *__restrict__ acc_out,
                               int *__restrict__ id_out, int *status, const uint64_t *__restrict__ key_in,
-                              uint64_t *__restrict__ key_out) {
+                              uint64_t *__restrict__ key_out, uint32_t *__restrict__ mask) {
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
+    mask[i] = 0u;  // for the build that follows
     uint32_t j = perm[i];
     if (j >= static_cast<uint64_t>(n)) {  // not a permutation: report, read in bounds
         record_error(status, NBODY_ERR_CAPACITY);
@@ -371,9 +368,19 @@ __device__ __forceinline__ int delta_at(const uint64_t *__restrict__ k, const in
     return base + 63 + __clz(static_cast<int>(i ^ j));                        // equal keys: break ties by index
 }
 
+// Also presets, for the kernels that follow, the scan's tile words, the child
+// table (two rows per thread: 2 n rows hold every record) and, with arrive set,
+// the climb's counters. n >= 1 threads.
 __global__ void radix_tree_kernel(const uint64_t *__restrict__ k, int64_t n, BinaryTree t, SegView sv,
-                                  uint32_t *__restrict__ mask, int base) {
+                                  uint32_t *__restrict__ mask, int base, unsigned long long *__restrict__ scan_words,
+                                  int scan_count, int4 *__restrict__ kids, unsigned *__restrict__ arrive) {
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    if (i < scan_count) scan_words[i] = 0ull;
+    const int4 none = make_int4(-1, -1, -1, -1);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) kids[4 * i + q] = none;
+    if (arrive) reinterpret_cast<uint2 *>(arrive)[i] = make_uint2(0u, 0u);
     if (i >= n - 1) return;
     const int *seg = sv.seg;
     const int dl = delta_at(k, seg, n, i, i - 1), dr = delta_at(k, seg, n, i, i + 1);
@@ -414,12 +421,98 @@ __global__ void radix_tree_kernel(const uint64_t *__restrict__ k, int64_t n, Bin
     if (top) atomicOr(&mask[lo], 1u << L);
 }
 
-__global__ void count_nodes_kernel(const uint64_t *__restrict__ k, int64_t n, const uint32_t *__restrict__ mask,
-                                   uint32_t *__restrict__ cnt, SegView sv) {
-    const int64_t b = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (b >= n) return;
-    const bool lone = !((b > 0 && same_key(k, sv, b, b - 1)) || (b + 1 < n && same_key(k, sv, b, b + 1)));
-    cnt[b] = __popc(mask[b]) + (lone ? 1u : 0u);
+// P[0 .. n] = exclusive prefix sums of cnt[b] = |mask[b]| + (b is a lone body),
+// P[n] = the number of records: one pass. A CTA takes the next tile (so that
+// every tile it waits on is already running), publishes its tile's count, adds
+// up the tiles before it 32 at a time until one that already knows its prefix
+// (bounded waits), and publishes its own prefix. words: [0] the tile counter,
+// then a word per tile, all zero before. As a count kernel and a three-kernel
+// scan this took 13 us and three launch gaps for any small n.
+constexpr int kScanThreads = 512;
+constexpr int kScanItems = 4;
+constexpr int kScanTile = kScanThreads * kScanItems;
+constexpr unsigned long long kScanCount = 1ull << 62, kScanPrefix = 2ull << 62, kScanValue = (1ull << 62) - 1ull;
+
+__global__ void __launch_bounds__(kScanThreads) count_scan_kernel(const uint64_t *__restrict__ k, int64_t n,
+                                                                  const uint32_t *__restrict__ mask, SegView sv,
+                                                                  uint32_t *__restrict__ P, unsigned long long *words,
+                                                                  int *status) {
+    __shared__ uint32_t warp_sums[kScanThreads / 32];
+    __shared__ unsigned s_tile;
+    __shared__ unsigned long long s_before;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) s_tile = static_cast<unsigned>(atomicAdd(&words[0], 1ull));
+    __syncthreads();
+    const unsigned tile = s_tile;
+    unsigned long long *word = words + 1;
+    const int64_t base = static_cast<int64_t>(tile) * kScanTile + threadIdx.x * kScanItems;
+    uint32_t v[kScanItems], run = 0;
+#pragma unroll
+    for (int j = 0; j < kScanItems; ++j) {
+        const int64_t b = base + j;
+        uint32_t c = 0;
+        if (b < n) {
+            const bool lone = !((b > 0 && same_key(k, sv, b, b - 1)) || (b + 1 < n && same_key(k, sv, b, b + 1)));
+            c = __popc(mask[b]) + (lone ? 1u : 0u);
+        }
+        v[j] = run;
+        run += c;
+    }
+    uint32_t x = run;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, off);
+        if (lane >= off) x += y;
+    }
+    if (lane == 31) warp_sums[warp] = x;
+    __syncthreads();
+    if (warp == 0) {
+        uint32_t s = lane < kScanThreads / 32 ? warp_sums[lane] : 0u;
+        const uint32_t own = s;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, s, off);
+            if (lane >= off) s += y;
+        }
+        const uint32_t all = __shfl_sync(0xffffffffu, s, 31);
+        if (lane < kScanThreads / 32) warp_sums[lane] = s - own;  // exclusive
+        volatile unsigned long long *vw = word;
+        if (lane == 0) vw[tile] = (tile == 0 ? kScanPrefix : kScanCount) | all;
+        unsigned long long before = 0;
+        for (int64_t at = static_cast<int64_t>(tile) - 1; at >= 0; at -= 32) {
+            const int64_t mine = at - lane;
+            unsigned long long w = kScanPrefix;  // in front of tile 0: nothing
+            if (mine >= 0) w = vw[mine];
+            if (!(w & ~kScanValue)) {
+                const unsigned long long t0 = global_ns();
+                for (uint32_t spin = 0; !((w = vw[mine]) & ~kScanValue);)
+                    if (++spin >= kWaitSpinCap || ((spin & 1023u) == 0 && global_ns() - t0 > kWaitLimitNs)) {
+                        record_error(status, NBODY_ERR_TIMEOUT);
+                        w = kScanPrefix;
+                        break;
+                    }
+            }
+            __syncwarp();
+            // The nearest tile with a prefix ends the look-back; the counts of those nearer count.
+            const unsigned known = __ballot_sync(0xffffffffu, (w & kScanPrefix) != 0ull);
+            const int last = known ? __ffs(known) - 1 : 31;
+            unsigned long long part = lane <= last ? w & kScanValue : 0ull;
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) part += __shfl_xor_sync(0xffffffffu, part, off);
+            before += part;
+            if (known) break;
+        }
+        if (lane == 0) {
+            if (tile > 0) vw[tile] = kScanPrefix | (before + all);
+            s_before = before;
+            if (static_cast<int64_t>(tile + 1) * kScanTile >= n) P[n] = static_cast<uint32_t>(before + all);
+        }
+    }
+    __syncthreads();
+    const uint32_t offset = static_cast<uint32_t>(s_before) + warp_sums[warp] + (x - run);
+#pragma unroll
+    for (int j = 0; j < kScanItems; ++j)
+        if (base + j < n) P[base + j] = v[j] + offset;
 }
 
 // Side^2 of the level-L cell holding `key`: the root box halved L times in
@@ -474,43 +567,38 @@ __device__ __forceinline__ int link_child(const BinaryTree &t, const uint32_t *_
     return par;
 }
 
-__global__ void emit_cells_kernel(const uint64_t *__restrict__ k, int64_t n, BinaryTree t,
-                                  const uint32_t *__restrict__ mask, const uint32_t *__restrict__ P,
-                                  const float *__restrict__ box, BHNode *__restrict__ nodes, Records r,
-                                  int *__restrict__ kids, SegView sv, bool parents) {
+// The records: thread i writes the cell whose top is radix-tree node i, and
+// body i's leaf if it is a lone body.
+__global__ void emit_kernel(const uint64_t *__restrict__ k, int64_t n, const float4 *__restrict__ pos, BinaryTree t,
+                            const uint32_t *__restrict__ mask, const uint32_t *__restrict__ P,
+                            const float *__restrict__ box, BHNode *__restrict__ nodes, Records r, int *__restrict__ kids,
+                            SegView sv, bool parents) {
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n - 1) return;
-    if (!t.top[i]) return;
+    if (i >= n) return;
     const int base = sv.seg ? 32 : 0;
-    const int L = level_c(t.delta[i], base);
-    const int lo = t.lo[i], hi = t.hi[i];
-    const int idx = record_of(t, mask, P, static_cast<int>(i), base);
-    int4 meta;
-    if (L < kMaxLevel) {
-        meta = make_int4(__float_as_int(cell_side2(k[lo], L, box_of(sv, box, lo))), static_cast<int>(P[hi + 1]), lo,
-                         0);
-    } else {  // bucket of bodies with identical keys: a leaf
-        meta = make_int4(__float_as_int(-1.f), static_cast<int>(P[hi + 1]), lo, hi - lo + 1);
+    if (i < n - 1 && t.top[i]) {
+        const int L = level_c(t.delta[i], base);
+        const int lo = t.lo[i], hi = t.hi[i];
+        const int idx = record_of(t, mask, P, static_cast<int>(i), base);
+        int4 meta;
+        if (L < kMaxLevel) {
+            meta = make_int4(__float_as_int(cell_side2(k[lo], L, box_of(sv, box, lo))), static_cast<int>(P[hi + 1]), lo,
+                             0);
+        } else {  // bucket of bodies with identical keys: a leaf
+            meta = make_int4(__float_as_int(-1.f), static_cast<int>(P[hi + 1]), lo, hi - lo + 1);
+        }
+        nodes[idx].meta = meta;
+        r.level[idx] = L;
+        const int par = i == 0 ? -1 : link_child(t, mask, P, t.iparent[i], base, k[lo], idx, kids);
+        if (parents) r.parent[idx] = par;  // for the climbing upsweep
     }
-    nodes[idx].meta = meta;
-    r.level[idx] = L;
-    const int par = i == 0 ? -1 : link_child(t, mask, P, t.iparent[i], base, k[lo], idx, kids);
-    if (parents) r.parent[idx] = par;  // for the climbing upsweep
-}
-
-__global__ void emit_leaves_kernel(const uint64_t *__restrict__ k, int64_t n, const float4 *__restrict__ pos,
-                                   BinaryTree t, const uint32_t *__restrict__ mask, const uint32_t *__restrict__ P,
-                                   BHNode *__restrict__ nodes, Records r, int *__restrict__ kids, SegView sv,
-                                   bool parents) {
-    const int64_t b = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (b >= n) return;
-    const bool lone = !((b > 0 && same_key(k, sv, b, b - 1)) || (b + 1 < n && same_key(k, sv, b, b + 1)));
+    const bool lone = !((i > 0 && same_key(k, sv, i, i - 1)) || (i + 1 < n && same_key(k, sv, i, i + 1)));
     if (!lone) return;
-    const int idx = static_cast<int>(P[b] + __popc(mask[b]));
-    nodes[idx].cm = pos[b];
-    nodes[idx].meta = make_int4(__float_as_int(-1.f), static_cast<int>(P[b + 1]), static_cast<int>(b), 1);
+    const int idx = static_cast<int>(P[i] + __popc(mask[i]));
+    nodes[idx].cm = pos[i];
+    nodes[idx].meta = make_int4(__float_as_int(-1.f), static_cast<int>(P[i + 1]), static_cast<int>(i), 1);
     r.level[idx] = kMaxLevel + 1;  // a lone body
-    const int par = n < 2 ? -1 : link_child(t, mask, P, t.lparent[b], sv.seg ? 32 : 0, k[b], idx, kids);
+    const int par = n < 2 ? -1 : link_child(t, mask, P, t.lparent[i], base, k[i], idx, kids);
     if (parents) r.parent[idx] = par;
 }
 
@@ -1226,94 +1314,6 @@ __global__ void unpermute_kernel(const int *__restrict__ ids, int64_t n, const f
     out[d] = v;
 }
 
-// exclusive scan of cnt[0..n) into P[0..n], P[n] = total (three phases).
-constexpr int kScanThreads = 1024;
-constexpr int kScanItems = 4;
-constexpr int kScanTile = kScanThreads * kScanItems;
-
-__global__ void __launch_bounds__(kScanThreads) scan_tiles_kernel(const uint32_t *__restrict__ in, int64_t n,
-                                                                  uint32_t *__restrict__ out,
-                                                                  uint32_t *__restrict__ tile_sums) {
-    __shared__ uint32_t warp_sums[32];
-    const int64_t base = static_cast<int64_t>(blockIdx.x) * kScanTile + threadIdx.x * kScanItems;
-    uint32_t v[kScanItems];
-    uint32_t run = 0;
-#pragma unroll
-    for (int j = 0; j < kScanItems; ++j) {
-        v[j] = base + j < n ? in[base + j] : 0u;
-        const uint32_t t2 = v[j];
-        v[j] = run;
-        run += t2;
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t x = run;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, x, off);
-        if (lane >= off) x += y;
-    }
-    if (lane == 31) warp_sums[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-        uint32_t w = warp_sums[lane];
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, w, off);
-            if (lane >= off) w += y;
-        }
-        warp_sums[lane] = w;
-    }
-    __syncthreads();
-    const uint32_t offset = (x - run) + (warp > 0 ? warp_sums[warp - 1] : 0u);
-#pragma unroll
-    for (int j = 0; j < kScanItems; ++j)
-        if (base + j < n) out[base + j] = v[j] + offset;
-    if (threadIdx.x == kScanThreads - 1) tile_sums[blockIdx.x] = offset + run;
-}
-
-__global__ void __launch_bounds__(1024) scan_sums_kernel(uint32_t *__restrict__ tile_sums, int tiles,
-                                                         uint32_t *__restrict__ total_out) {
-    __shared__ uint32_t carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (int base = 0; base < tiles; base += 1024) {
-        const int i = base + threadIdx.x;
-        const uint32_t v = i < tiles ? tile_sums[i] : 0u;
-        uint32_t x = v;
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, x, off);
-            if (lane >= off) x += y;
-        }
-        __shared__ uint32_t ws[32];
-        if (lane == 31) ws[warp] = x;
-        __syncthreads();
-        if (warp == 0) {
-            uint32_t w = ws[lane];
-#pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, w, off);
-                if (lane >= off) w += y;
-            }
-            ws[lane] = w;
-        }
-        __syncthreads();
-        const uint32_t incl = x + (warp > 0 ? ws[warp - 1] : 0u);
-        if (i < tiles) tile_sums[i] = carry + incl - v;
-        __syncthreads();
-        if (threadIdx.x == 1023) carry += incl;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) *total_out = carry;
-}
-
-__global__ void scan_add_kernel(uint32_t *__restrict__ out, int64_t n, const uint32_t *__restrict__ tile_sums) {
-    const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    out[i] += tile_sums[i / kScanTile];
-}
-
 unsigned grid_for(int64_t n, int threads) { return static_cast<unsigned>((n + threads - 1) / threads); }
 
 // Depth of the reference's fully expanded top levels for n bodies
@@ -1372,9 +1372,8 @@ size_t bh_workspace_layout(int64_t n, void *base, BHWorkspace *w) {
     w->rec.list = w->rec.arrive;  // one schedule or the other per build
     w->rec.lvl = static_cast<unsigned *>(take(sizeof(unsigned) * 96));
     w->mask = static_cast<uint32_t *>(take(sizeof(uint32_t) * nn));
-    w->cnt = static_cast<uint32_t *>(take(sizeof(uint32_t) * nn));
     w->P = static_cast<uint32_t *>(take(sizeof(uint32_t) * (nn + 1)));
-    w->scan_sums = static_cast<uint32_t *>(take(sizeof(uint32_t) * static_cast<size_t>(tiles + 1)));
+    w->scan_words = static_cast<unsigned long long *>(take(sizeof(unsigned long long) * static_cast<size_t>(tiles + 1)));
     w->nodes = static_cast<BHNode *>(take(sizeof(BHNode) * 2 * nn));
     w->kids = static_cast<int *>(take(sizeof(int) * 8 * 2 * nn));
     w->counter_mem = static_cast<unsigned long long *>(take(sizeof(unsigned long long) * 2));
@@ -1421,7 +1420,7 @@ cudaError_t bh_gather(int64_t n, const BHWorkspace &w, const float4 *pos_in, con
                       int *id_out, cudaStream_t st, int *status, StageTimer *timer) {
     if (timer) timer->begin(kStageGather, st);
     gather_kernel<<<grid_for(n, 256), 256, 0, st>>>(w.vals[0], n, pos_in, vel_in, acc_in, id_in, pos_out, vel_out,
-                                                    acc_out, id_out, status, nullptr, nullptr);
+                                                    acc_out, id_out, status, nullptr, nullptr, w.mask);
     if (timer) timer->end(kStageGather, st);
     return cudaGetLastError();
 }
@@ -1444,28 +1443,18 @@ cudaError_t bh_build(const float4 *pos_sorted, int64_t n, BHWorkspace &w, cudaSt
                      StageTimer *timer, const SegView &sv) {
     if (timer) timer->begin(kStageBuild, st);
     const uint64_t *k = w.keys[0];
-    cudaError_t e = cudaMemsetAsync(w.mask, 0, sizeof(uint32_t) * static_cast<size_t>(n), st);
-    if (e != cudaSuccess) return e;
-    if (n >= 2) {
-        radix_tree_kernel<<<grid_for(n - 1, 256), 256, 0, st>>>(k, n, w.tree, sv, w.mask, sv.seg ? 32 : 0);
-    }
-    count_nodes_kernel<<<grid_for(n, 256), 256, 0, st>>>(k, n, w.mask, w.cnt, sv);
-    const int tiles = static_cast<int>((n + kScanTile - 1) / kScanTile);
-    scan_tiles_kernel<<<tiles, kScanThreads, 0, st>>>(w.cnt, n, w.P, w.scan_sums);
-    scan_sums_kernel<<<1, 1024, 0, st>>>(w.scan_sums, tiles, w.P + n);
-    scan_add_kernel<<<grid_for(n, 256), 256, 0, st>>>(w.P, n, w.scan_sums);
     const bool levels = bh_upsweep_by_levels(n, sv.seg != nullptr);
     // Records: at most 2n (n - 1 cells and n leaves).
     const int64_t cap = 2 * (n > 1 ? n : 2);
-    e = cudaMemsetAsync(w.kids, 0xff, sizeof(int) * 8 * static_cast<size_t>(cap), st);
-    if (e == cudaSuccess && !levels)
-        e = cudaMemsetAsync(w.rec.arrive, 0, sizeof(unsigned) * static_cast<size_t>(cap), st);
+    const int tiles = static_cast<int>((n + kScanTile - 1) / kScanTile);
+    radix_tree_kernel<<<grid_for(n, 256), 256, 0, st>>>(k, n, w.tree, sv, w.mask, sv.seg ? 32 : 0, w.scan_words, tiles + 1,
+                                                        reinterpret_cast<int4 *>(w.kids),
+                                                        levels ? nullptr : w.rec.arrive);
+    count_scan_kernel<<<tiles, kScanThreads, 0, st>>>(k, n, w.mask, sv, w.P, w.scan_words, status);
+    emit_kernel<<<grid_for(n, 256), 256, 0, st>>>(k, n, pos_sorted, w.tree, w.mask, w.P, w.box, w.nodes, w.rec, w.kids, sv,
+                                                  !levels);
+    cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    if (n >= 2)
-        emit_cells_kernel<<<grid_for(n - 1, 256), 256, 0, st>>>(k, n, w.tree, w.mask, w.P, w.box, w.nodes, w.rec,
-                                                                w.kids, sv, !levels);
-    emit_leaves_kernel<<<grid_for(n, 256), 256, 0, st>>>(k, n, pos_sorted, w.tree, w.mask, w.P, w.nodes, w.rec,
-                                                         w.kids, sv, !levels);
     if (timer) timer->end(kStageBuild, st);
     if (timer) timer->begin(kStageUpsweep, st);
     if (!levels) {
@@ -1632,7 +1621,8 @@ cudaError_t bh_ensemble_step(int64_t n, BHWorkspace &w, const BHEnsembleTables &
     if (tm) tm->begin(kStageGather, st);
     // Sorted keys into keys[0] (the build reads them there), permutation in vals[0].
     uint64_t *ksorted = w.keys[0];
-    gather_kernel<<<grid_for(n, 256), 256, 0, st>>>(v0, n, P, V, A, I, Po, Vo, Ao, Io, status, e.keys_orig, ksorted);
+    gather_kernel<<<grid_for(n, 256), 256, 0, st>>>(v0, n, P, V, A, I, Po, Vo, Ao, Io, status, e.keys_orig, ksorted,
+                                                    w.mask);
     if (tm) tm->end(kStageGather, st);
     err = cudaGetLastError();
     if (err != cudaSuccess) return err;

@@ -68,9 +68,8 @@ struct BHWorkspace {
     BinaryTree tree{};
     Records rec{};
     uint32_t *mask = nullptr;
-    uint32_t *cnt = nullptr;
     uint32_t *P = nullptr;  // n + 1 entries; P[n] = record count
-    uint32_t *scan_sums = nullptr;
+    unsigned long long *scan_words = nullptr;
     BHNode *nodes = nullptr;  // up to 2n records
     int *kids = nullptr;      // child table: 8 places per cell record, by key digit; -1: no child
     // Traversal counters (pairwise evaluations, warp record visits): the

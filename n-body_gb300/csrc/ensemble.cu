@@ -785,12 +785,12 @@ int nbody_ensemble_counts(nbody_ensemble *e, int *systems, int64_t *pp_bodies, i
     if (bh_bodies) *bh_bodies = e->bh_n;
     if (launches_per_step) {
         // direct sum: 1; Barnes-Hut: bbox, keys, sort by key, segment keys and
-        // sort by segment, gather, 7 build kernels, the upsweep's, one walk per
+        // sort by segment, gather, 3 build kernels, the upsweep's, one walk per
         // team size
         int l = e->pp_nitems > 0 ? 1 : 0;
         if (e->bh_n > 0)
             l += 2 + nbody::sort_launches(e->bh_n) +
-                 (e->tab.systems > 1 ? 1 + nbody::sort_launches(e->bh_n, e->tab.seg_passes) : 0) + 1 + 7 +
+                 (e->tab.systems > 1 ? 1 + nbody::sort_launches(e->bh_n, e->tab.seg_passes) : 0) + 1 + 3 +
                  nbody::bh_upsweep_launches(e->bh_n, true) + static_cast<int>(e->tab.teams.size());
         *launches_per_step = l;
     }

@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <initializer_list>
 #include <new>
 #include <string>
 #include <vector>
@@ -59,8 +60,16 @@ struct nbody_ctx {
     float4 *vel = nullptr;
     float4 *acc = nullptr;
     float4 *stage = nullptr;  // 2n float4: reference-layout positions, then masses
-    int *status = nullptr;    // device status word
-    int *status_host = nullptr;  // page-locked copy of it, read after a stream sync
+    // Status word that kernels raise: page-locked host memory mapped into the
+    // device (status_host its host address), so that reading it takes a wait
+    // for the stream and no copy; device memory where that cannot be had.
+    int *status = nullptr;
+    int *status_host = nullptr;
+    // Page-locked stand-ins for the pageable arrays of a small system (five
+    // arrays of n float4; made on first use).
+    float4 *bounce = nullptr;
+    bool bounce_failed = false;
+    bool bounce_read = false;  // work on the stream may still read it
     void *scratch = nullptr;
     size_t scratch_bytes = 0;
     size_t scratch_arrivals = 0;  // bytes of arrival counters of the plan that used it last
@@ -162,15 +171,15 @@ int ensure_scratch(nbody_ctx *ctx, int64_t n, nbody::PPPlan &plan) {
 int read_status(nbody_ctx *ctx) {
     int h = NBODY_OK;
     if (ctx->status_host) {
-        NB_CK(ctx, cudaMemcpyAsync(ctx->status_host, ctx->status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-        NB_CK(ctx, cudaMemsetAsync(ctx->status, 0, sizeof(int), ctx->stream));
         NB_CK(ctx, cudaStreamSynchronize(ctx->stream));
-        h = *ctx->status_host;
+        h = *static_cast<volatile int *>(ctx->status_host);
+        if (h != NBODY_OK) *static_cast<volatile int *>(ctx->status_host) = NBODY_OK;
     } else {
         NB_CK(ctx, cudaMemcpyAsync(&h, ctx->status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
         NB_CK(ctx, cudaMemsetAsync(ctx->status, 0, sizeof(int), ctx->stream));
         NB_CK(ctx, cudaStreamSynchronize(ctx->stream));
     }
+    ctx->bounce_read = false;
     if (h != NBODY_OK && ctx->scratch) {
         // A kernel gave up part-way: its arrival counters may be left non-zero.
         NB_CK(ctx, cudaMemsetAsync(ctx->scratch, 0, ctx->scratch_bytes, ctx->stream));
@@ -343,6 +352,72 @@ int replay(nbody_ctx *ctx, StepGraph &g, const GraphKey &key, Body &&body, bool 
     return NBODY_OK;
 }
 
+// A pageable array costs a copy through the driver's own staging each way (some
+// 12 us whatever its size) and rules out the in-place kernels and the graph of
+// the host call. Up to this many bodies the caller's pageable arrays are copied
+// into page-locked stand-ins by the host instead (16 bytes per body and array),
+// and the call runs on those. GB300, one host step with pageable arrays, us,
+// before / after: direct sum of 1,000 bodies 97 / 43, of 4,096 109 / 54, Barnes-Hut
+// of 4,096 250 / 160. The host copies 24 GB/s, 85 us of a call at 16,384 bodies, where
+// the driver takes 80 (direct sum) to 150; at 32,768 its 80 to 170 win.
+constexpr int64_t kBounceBodies = 16384;
+
+// Whether the arrays (some may be null) all lie in pageable memory, so that
+// they may be copied by the host: none begins or ends in page-locked or device
+// memory, whose copies the driver checks.
+bool pageable(std::initializer_list<const void *> arrays, size_t bytes) {
+    for (const void *p : arrays) {
+        if (!p) continue;
+        for (const char *q : {static_cast<const char *>(p), static_cast<const char *>(p) + bytes - 1}) {
+            cudaPointerAttributes a;
+            if (cudaPointerGetAttributes(&a, q) != cudaSuccess) {
+                cudaGetLastError();
+                return false;
+            }
+            if (a.type != cudaMemoryTypeUnregistered) return false;
+        }
+    }
+    return true;
+}
+
+// Whether a call on these arrays takes the stand-ins (made, and free to be
+// written, when it does).
+bool use_bounce(nbody_ctx *ctx, std::initializer_list<const void *> arrays) {
+    if (ctx->n > kBounceBodies || ctx->bounce_failed) return false;
+    const size_t b4 = static_cast<size_t>(ctx->n) * sizeof(float4);
+    if (!pageable(arrays, b4)) return false;
+    if (!ctx->bounce) {
+        if (cudaHostAlloc(reinterpret_cast<void **>(&ctx->bounce), 5 * b4, cudaHostAllocMapped) != cudaSuccess) {
+            cudaGetLastError();
+            ctx->bounce = nullptr;
+            ctx->bounce_failed = true;
+            return false;
+        }
+    }
+    if (ctx->bounce_read && cudaStreamSynchronize(ctx->stream) != cudaSuccess) return false;
+    ctx->bounce_read = false;
+    return true;
+}
+
+float *bounce_in(nbody_ctx *ctx, int slot, const float *from) {
+    if (!from) return nullptr;
+    float4 *to = ctx->bounce + slot * ctx->n;
+    std::memcpy(to, from, static_cast<size_t>(ctx->n) * sizeof(float4));
+    return reinterpret_cast<float *>(to);
+}
+
+float *bounce_slot(nbody_ctx *ctx, int slot, const float *wanted) {
+    return wanted ? reinterpret_cast<float *>(ctx->bounce + slot * ctx->n) : nullptr;
+}
+
+void bounce_out(nbody_ctx *ctx, int slot, float *to) {
+    if (to) std::memcpy(to, ctx->bounce + slot * ctx->n, static_cast<size_t>(ctx->n) * sizeof(float4));
+}
+
+// Whether a call that returned rc has written its outputs (a kernel's status is
+// reported after the results are out).
+bool has_outputs(int rc) { return rc == NBODY_OK || rc == NBODY_ERR_CAPACITY || rc == NBODY_ERR_TIMEOUT; }
+
 // Steps on the resident state. From the second step after an upload (ids
 // valid, the same launches every step) each step is one graph launch, one
 // graph per parity of the velocity buffers: one host call instead of some
@@ -412,11 +487,8 @@ int nbody_create(nbody_ctx **out, int device, int mode, int64_t n, float dt, flo
     alloc(reinterpret_cast<void **>(&ctx->vel), b4);
     alloc(reinterpret_cast<void **>(&ctx->acc), b4);
     alloc(reinterpret_cast<void **>(&ctx->stage), 2 * b4);
-    alloc(reinterpret_cast<void **>(&ctx->status), sizeof(int));
-    if (rc == NBODY_OK && cudaMallocHost(reinterpret_cast<void **>(&ctx->status_host), sizeof(int)) != cudaSuccess) {
-        cudaGetLastError();  // the status is then read into pageable memory
-        ctx->status_host = nullptr;
-    }
+    if (rc == NBODY_OK) ctx->status_host = nbody::mapped_word(&ctx->status);
+    if (!ctx->status_host) alloc(reinterpret_cast<void **>(&ctx->status), sizeof(int));
     if (mode == NBODY_MODE_BH) {
         ctx->vel2[0] = ctx->vel;
         ctx->acc2[0] = ctx->acc;
@@ -432,7 +504,7 @@ int nbody_create(nbody_ctx **out, int device, int mode, int64_t n, float dt, flo
     }
     if (rc == NBODY_OK && mode == NBODY_MODE_BH) rc = ensure_workspace(ctx, n);
     if (rc == NBODY_OK) {
-        cudaError_t e = cudaMemsetAsync(ctx->status, 0, sizeof(int), ctx->stream);
+        cudaError_t e = ctx->status_host ? cudaSuccess : cudaMemsetAsync(ctx->status, 0, sizeof(int), ctx->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess) rc = fail(ctx, e);
     }
@@ -454,8 +526,9 @@ int nbody_destroy(nbody_ctx *ctx) {
         cudaFree(ctx->vel);
         cudaFree(ctx->acc);
         cudaFree(ctx->stage);
-        cudaFree(ctx->status);
         if (ctx->status_host) cudaFreeHost(ctx->status_host);
+        else cudaFree(ctx->status);
+        if (ctx->bounce) cudaFreeHost(ctx->bounce);
         cudaFree(ctx->scratch);
         cudaFree(ctx->vel2[1]);
         cudaFree(ctx->acc2[1]);
@@ -492,6 +565,13 @@ int nbody_upload(nbody_ctx *ctx, const float *positions4, const float *velocitie
     if (!ctx || !positions4 || !masses4) return NBODY_ERR_ARG;
     DeviceGuard dg(ctx->device);
     const size_t b4 = static_cast<size_t>(ctx->n) * sizeof(float4);
+    if (use_bounce(ctx, {positions4, velocities4, accelerations4, masses4})) {
+        positions4 = bounce_in(ctx, 0, positions4);
+        velocities4 = bounce_in(ctx, 1, velocities4);
+        accelerations4 = bounce_in(ctx, 2, accelerations4);
+        masses4 = bounce_in(ctx, 3, masses4);
+        ctx->bounce_read = true;
+    }
     // Page-locked host buffers are read in place by one kernel; otherwise one
     // copy per array into the staging area, then the pack kernel.
     const float4 *mp = nbody::host_mapped(positions4, b4, ctx->device);
@@ -535,6 +615,18 @@ int nbody_download(nbody_ctx *ctx, float *positions4, float *velocities4, float 
     DeviceGuard dg(ctx->device);
     const size_t b4 = static_cast<size_t>(ctx->n) * sizeof(float4);
     const int64_t n = ctx->n;
+    if ((positions4 || velocities4 || accelerations4 || forces4) &&
+        use_bounce(ctx, {positions4, velocities4, accelerations4, forces4})) {
+        const int rc = nbody_download(ctx, bounce_slot(ctx, 0, positions4), bounce_slot(ctx, 1, velocities4),
+                                      bounce_slot(ctx, 2, accelerations4), bounce_slot(ctx, 4, forces4));
+        if (has_outputs(rc)) {
+            bounce_out(ctx, 0, positions4);
+            bounce_out(ctx, 1, velocities4);
+            bounce_out(ctx, 2, accelerations4);
+            bounce_out(ctx, 4, forces4);
+        }
+        return rc;
+    }
     {
         // Page-locked host buffers are written in place by one kernel, in the
         // caller's order (through the inverse of the sorted order, built in the
@@ -733,6 +825,21 @@ bool pp_update_graphed(nbody_ctx *ctx, const float *positions4, float *velocitie
 int nbody_update_host(nbody_ctx *ctx, float *positions4, float *velocities4, float *accelerations4,
                       const float *masses4, float *forces4, int steps) {
     if (!ctx || !positions4 || !velocities4 || !accelerations4 || !masses4 || steps < 0) return NBODY_ERR_ARG;
+    {
+        DeviceGuard dg(ctx->device);
+        if (use_bounce(ctx, {positions4, velocities4, accelerations4, masses4, forces4})) {
+            const int rc = nbody_update_host(ctx, bounce_in(ctx, 0, positions4), bounce_in(ctx, 1, velocities4),
+                                             bounce_in(ctx, 2, accelerations4), bounce_in(ctx, 3, masses4),
+                                             bounce_slot(ctx, 4, forces4), steps);
+            if (has_outputs(rc)) {
+                bounce_out(ctx, 0, positions4);
+                bounce_out(ctx, 1, velocities4);
+                bounce_out(ctx, 2, accelerations4);
+                bounce_out(ctx, 4, forces4);
+            }
+            return rc;
+        }
+    }
     if (ctx->mode == NBODY_MODE_PP && steps == 1) {
         int rc = NBODY_OK;
         if (pp_update_graphed(ctx, positions4, velocities4, accelerations4, masses4, forces4, &rc)) return rc;

@@ -82,7 +82,8 @@ struct nbody_ensemble {
     cudaStream_t own_stream = nullptr, stream = nullptr, side = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
     cudaMemPool_t pool = nullptr;
-    int *status = nullptr;
+    int *status = nullptr;       // raised by kernels: page-locked host memory (status_host its
+    int *status_host = nullptr;  // host address) mapped into the device, or device memory
     std::string last_error;
     std::vector<Sys> sys;
     bool dirty = true;
@@ -191,11 +192,17 @@ void clear_graphs(nbody_ensemble *e) {
 
 int read_status(nbody_ensemble *e) {
     int h = 0;
-    EN_CK(e, cudaMemcpyAsync(&h, e->status, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
-    EN_CK(e, cudaStreamSynchronize(e->stream));
+    if (e->status_host) {
+        EN_CK(e, cudaStreamSynchronize(e->stream));
+        h = *static_cast<volatile int *>(e->status_host);
+    } else {
+        EN_CK(e, cudaMemcpyAsync(&h, e->status, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
+        EN_CK(e, cudaStreamSynchronize(e->stream));
+    }
     if (h != NBODY_OK) {
         // Re-arm everything a failed kernel may have left half way.
-        cudaMemsetAsync(e->status, 0, sizeof(int), e->stream);
+        if (e->status_host) *static_cast<volatile int *>(e->status_host) = NBODY_OK;
+        else cudaMemsetAsync(e->status, 0, sizeof(int), e->stream);
         if (e->pp_sched) cudaMemsetAsync(e->pp_sched, 0, 2 * sizeof(unsigned), e->stream);
         if (e->tab.systems > 0) nbody::bh_seed_boxes(e->tab, e->stream);
         cudaStreamSynchronize(e->stream);
@@ -506,8 +513,11 @@ int nbody_ensemble_create(nbody_ensemble **out, int device, int64_t crossover) {
         uint64_t keep = UINT64_MAX;  // keep freed blocks for the next layout
         if (rc == NBODY_OK) ck(cudaMemPoolSetAttribute(e->pool, cudaMemPoolAttrReleaseThreshold, &keep));
     }
-    ck(cudaMalloc(&e->status, sizeof(int)));
-    if (rc == NBODY_OK) ck(cudaMemsetAsync(e->status, 0, sizeof(int), e->stream));
+    if (rc == NBODY_OK) e->status_host = nbody::mapped_word(&e->status);
+    if (!e->status_host) {
+        ck(cudaMalloc(&e->status, sizeof(int)));
+        if (rc == NBODY_OK) ck(cudaMemsetAsync(e->status, 0, sizeof(int), e->stream));
+    }
     if (rc == NBODY_OK) ck(nbody::sort_prepare(device));
     if (rc == NBODY_OK) ck(cudaStreamSynchronize(e->stream));
     if (rc != NBODY_OK) {
@@ -532,7 +542,8 @@ int nbody_ensemble_destroy(nbody_ensemble *e) {
             cudaStreamSynchronize(e->stream);
         }
         if (e->pool) cudaMemPoolDestroy(e->pool);
-        if (e->status) cudaFree(e->status);
+        if (e->status_host) cudaFreeHost(e->status_host);
+        else if (e->status) cudaFree(e->status);
         if (e->fork) cudaEventDestroy(e->fork);
         if (e->join) cudaEventDestroy(e->join);
         if (e->side) cudaStreamDestroy(e->side);

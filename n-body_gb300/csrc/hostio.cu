@@ -135,6 +135,19 @@ float4 *host_mapped(const void *p, size_t bytes, int device) {
     return static_cast<float4 *>(a.devicePointer);
 }
 
+int *mapped_word(int **device) {
+    int *host = nullptr;
+    if (cudaHostAlloc(reinterpret_cast<void **>(&host), sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
+        cudaHostGetDevicePointer(reinterpret_cast<void **>(device), host, 0) != cudaSuccess) {
+        cudaGetLastError();
+        if (host) cudaFreeHost(host);
+        *device = nullptr;
+        return nullptr;
+    }
+    *host = 0;
+    return host;
+}
+
 cudaError_t merge_masses(float4 *pos_mass, const float4 *masses4, int64_t n, cudaStream_t stream) {
     if (n <= 0) return cudaSuccess;
     const int threads = 256;

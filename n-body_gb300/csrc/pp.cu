@@ -418,15 +418,39 @@ DeviceInfo device_info(int device) {
 // cost and the second kernel outweigh the operations saved.
 constexpr int64_t kSymMinBodies = 10000;
 
+// A forced shape of the kernels over ordered pairs.
+bool pp_shape_forced() {
+    return std::getenv("NBODY_PP_K") || std::getenv("NBODY_PP_THREADS") || std::getenv("NBODY_PP_SLICES") ||
+           std::getenv("NBODY_PP_LINEAR");
+}
+
 // Every pair once (pp_sym.cu) or every ordered pair: forced by NBODY_PP_SYM = 1
-// / 0; a forced shape of the latter (NBODY_PP_K, _THREADS, _SLICES, _LINEAR)
-// rules the former out.
+// / 0; a forced shape of the latter rules the former out.
 bool pp_sym_wanted(int64_t n) {
-    if (std::getenv("NBODY_PP_K") || std::getenv("NBODY_PP_THREADS") || std::getenv("NBODY_PP_SLICES") ||
-        std::getenv("NBODY_PP_LINEAR"))
-        return false;
+    if (pp_shape_forced()) return false;
     if (const char *e = std::getenv("NBODY_PP_SYM")) return std::atoi(e) == 1;
     return n >= kSymMinBodies;
+}
+
+// Below 8,192 bodies what counts is how long one CTA takes, not how full the
+// CTAs are: one body per thread and short j-slices put every SM to work early,
+// from some 4,000 bodies on four bodies per thread in one CTA per SM (two
+// where its slices would leave most of the second half of them idle). Sweep of
+// K x T x slices on GB300 (us, two bodies per thread as before / this rule): 256
+// bodies 8.3 / 6.2, 512 14.4 / 7.3, 1,000 18.5 / 8.2, 2,000 16.5 / 10.3, 3,000 16.5 /
+// 12.4, 4,000 16.5 / 14.4, 5,003 24.8 / 18.5, 6,500 33 / 26, 7,000 33 / 27, 8,000 37 / 31.
+constexpr int64_t kSmallBodies = 8192;
+
+void pp_small_shape(int64_t n, int64_t sms, PPPlan *p) {
+    p->k = n < 3750 ? 1 : 4;
+    p->threads = n < 6750 ? 128 : 256;
+    const int64_t per_block = static_cast<int64_t>(p->threads) * p->k;
+    p->iblocks = static_cast<int>((n + per_block - 1) / per_block);
+    int64_t s;
+    if (n < 3750) s = n < 1536 ? (n + 32) / 64 : (n + 56) / 112;  // j-bodies per slice
+    else if (n < 6250 || p->threads == 256) s = sms / p->iblocks;
+    else s = 2 * sms / p->iblocks;
+    p->slices = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(s, 64)));
 }
 
 int k_index(int k) { return k == 1 ? 0 : k == 2 ? 1 : k == 4 ? 2 : 3; }
@@ -447,10 +471,19 @@ PPPlan pp_plan(int64_t n, int device, bool allow_linear, bool allow_sym) {
             return p;
         }
     }
+    if (n < kSmallBodies && !pp_shape_forced()) {
+        pp_small_shape(n, d.sms > 0 ? d.sms : 1, &p);
+        if (p.slices > 1) {
+            p.arrivals_bytes = (static_cast<size_t>(p.iblocks) * sizeof(unsigned) + 255) & ~static_cast<size_t>(255);
+            p.partial_bytes =
+                p.arrivals_bytes + static_cast<size_t>(p.slices) * static_cast<size_t>(n) * sizeof(float4);
+        }
+        return p;
+    }
     // Default shapes from sweeps on GB300 (T x K in {128, 256} x {1, 2, 4, 8},
     // N = 4,096 ... 131,072): from N = 8,192 on, 256 threads with 4 i-bodies
-    // each (one CTA per SM at 140 registers, ILP-bound) is fastest; below it 2
-    // i-bodies per thread give the j-slicing enough CTAs.
+    // each (one CTA per SM at 140 registers, ILP-bound) is fastest; a forced
+    // shape below it starts from 2 i-bodies per thread.
     int k = n >= 8192 ? 4 : 2;
     if (const char *e = std::getenv("NBODY_PP_K")) {
         const int v = std::atoi(e);

@@ -44,6 +44,7 @@
 #include "bh.h"
 #include "bh_walk.cuh"
 #include "common.cuh"
+#include "launch.h"
 #include "sort.h"
 
 namespace nbody {
@@ -104,6 +105,7 @@ __device__ __forceinline__ void block_box(float (&mn)[3], float (&mx)[3], float 
 
 __global__ void bbox_kernel(const float4 *__restrict__ pos, int64_t n, float *__restrict__ partial,
                             unsigned *__restrict__ counter, float *__restrict__ box) {
+    wait_for_launches_before();
     __shared__ float wm[32][6];
     __shared__ bool last;
     float mn[3] = {FLT_MAX, FLT_MAX, FLT_MAX};
@@ -209,6 +211,7 @@ __device__ __forceinline__ uint64_t octree_key(float px, float py, float pz, con
 template <int MODE>
 __global__ void morton_kernel(const float4 *__restrict__ pos, int64_t n, const float *__restrict__ box,
                               uint64_t *__restrict__ keys, uint32_t *__restrict__ vals) {
+    wait_for_launches_before();
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 p = pos[i];
@@ -230,6 +233,7 @@ __global__ void morton_kernel(const float4 *__restrict__ pos, int64_t n, const f
 __global__ void __launch_bounds__(256) bbox_seg_kernel(const float4 *__restrict__ pos,
                                                        const int4 *__restrict__ chunks,
                                                        unsigned *__restrict__ acc, float *__restrict__ boxes) {
+    wait_for_launches_before();
     const int4 c = chunks[blockIdx.x];
     float mn[3] = {FLT_MAX, FLT_MAX, FLT_MAX};
     float mx[3] = {FLT_MIN, FLT_MIN, FLT_MIN};
@@ -300,6 +304,7 @@ template <int MODE>
 __global__ void keys_seg_kernel(const float4 *__restrict__ pos, int64_t n, const int *__restrict__ seg,
                                 const float *__restrict__ boxes, uint64_t *__restrict__ keys,
                                 uint64_t *__restrict__ keys_orig, uint32_t *__restrict__ vals) {
+    wait_for_launches_before();
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 p = pos[i];
@@ -338,6 +343,8 @@ __global__ void gather_kernel(const uint32_t *__restrict__ perm, int64_t n, cons
                               float4 *__restrict__ vel_out, float4 *__restrict__ acc_out,
                               int *__restrict__ id_out, int *status, const uint64_t *__restrict__ key_in,
                               uint64_t *__restrict__ key_out, uint32_t *__restrict__ mask) {
+    wait_for_launches_before();
+    wait_for_launches_before();
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
     mask[i] = 0u;  // for the build that follows
@@ -374,6 +381,7 @@ __device__ __forceinline__ int delta_at(const uint64_t *__restrict__ k, const in
 __global__ void radix_tree_kernel(const uint64_t *__restrict__ k, int64_t n, BinaryTree t, SegView sv,
                                   uint32_t *__restrict__ mask, int base, unsigned long long *__restrict__ scan_words,
                                   int scan_count, int4 *__restrict__ kids, unsigned *__restrict__ arrive) {
+    wait_for_launches_before();
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
     if (i < scan_count) scan_words[i] = 0ull;
@@ -437,6 +445,7 @@ __global__ void __launch_bounds__(kScanThreads) count_scan_kernel(const uint64_t
                                                                   const uint32_t *__restrict__ mask, SegView sv,
                                                                   uint32_t *__restrict__ P, unsigned long long *words,
                                                                   int *status) {
+    wait_for_launches_before();
     __shared__ uint32_t warp_sums[kScanThreads / 32];
     __shared__ unsigned s_tile;
     __shared__ unsigned long long s_before;
@@ -573,6 +582,7 @@ __global__ void emit_kernel(const uint64_t *__restrict__ k, int64_t n, const flo
                             const uint32_t *__restrict__ mask, const uint32_t *__restrict__ P,
                             const float *__restrict__ box, BHNode *__restrict__ nodes, Records r, int *__restrict__ kids,
                             SegView sv, bool parents) {
+    wait_for_launches_before();
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int base = sv.seg ? 32 : 0;
@@ -711,6 +721,7 @@ __global__ void upsweep_climb_kernel(const uint64_t *__restrict__ k, int64_t n, 
                                      const uint32_t *__restrict__ mask, const uint32_t *__restrict__ P,
                                      BHNode *nodes, Records r, const int *__restrict__ kids, int father_depth,
                                      int *status, SegView sv) {
+    wait_for_launches_before();
     const int64_t b = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (b >= n) return;
     if (sv.seg) father_depth = sv.fdepth[sv.seg[b]];
@@ -748,6 +759,7 @@ __global__ void upsweep_climb_kernel(const uint64_t *__restrict__ k, int64_t n, 
 __global__ void bucket_cm_kernel(const uint64_t *__restrict__ k, int64_t n, const float4 *__restrict__ pos,
                                  const uint32_t *__restrict__ mask, const uint32_t *__restrict__ P,
                                  BHNode *__restrict__ nodes, SegView sv) {
+    wait_for_launches_before();
     const int64_t b = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (b >= n) return;
     const bool left_eq = b > 0 && same_key(k, sv, b, b - 1);
@@ -760,6 +772,7 @@ __global__ void bucket_cm_kernel(const uint64_t *__restrict__ k, int64_t n, cons
 // Cells per octree level (levels 0 .. kMaxLevel - 1) over records [0, *total).
 __global__ void level_count_kernel(const int *__restrict__ level, const uint32_t *__restrict__ total,
                                    unsigned *__restrict__ lvl) {
+    wait_for_launches_before();
     __shared__ unsigned h[kMaxLevel];
     if (threadIdx.x < kMaxLevel) h[threadIdx.x] = 0u;
     __syncthreads();
@@ -779,6 +792,7 @@ __global__ void level_count_kernel(const int *__restrict__ level, const uint32_t
 __global__ void level_scatter_kernel(const int *__restrict__ level, const uint32_t *__restrict__ total,
                                      unsigned *__restrict__ lvl, unsigned *__restrict__ list, int64_t cap,
                                      int *status) {
+    wait_for_launches_before();
     __shared__ unsigned h[kMaxLevel], base[kMaxLevel], off[kMaxLevel];
     if (threadIdx.x == 0) {
         unsigned run = 0;
@@ -813,6 +827,7 @@ __global__ void __launch_bounds__(256, 4)
     level_cm_kernel(int L, BHNode *nodes, const int *__restrict__ level, const int *__restrict__ kids,
                     const unsigned *__restrict__ list, const unsigned *__restrict__ lvl,
                     int father_depth, SegView sv) {
+    wait_for_launches_before();
     const unsigned count = lvl[L], first = lvl[32 + L];
     const unsigned stride = gridDim.x * blockDim.x;
     for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += stride) {
@@ -1046,6 +1061,7 @@ __global__ void __launch_bounds__(64, (COUNT || SEG) ? 16 : 24) cell_walk_kernel
     float4 *__restrict__ vel, float4 *__restrict__ acc, float4 *__restrict__ force_out, const int *__restrict__ ids,
     unsigned long long *__restrict__ counters, float *__restrict__ phi_out, int euler, const int4 *__restrict__ work,
     int nwork, const float4 *__restrict__ params, const uint32_t *__restrict__ P, const HostOut host) {
+    wait_for_launches_before();
     // One block of shared memory per warp, addressed from one base.
     struct __align__(16) WarpArea {
         int4 stk_i[kCellDepth];     // cell, mask A, mask B, box hz (float bits)
@@ -1387,7 +1403,7 @@ cudaError_t bh_bbox(const float4 *pos, int64_t n, BHWorkspace &w, cudaStream_t s
     int blocks = static_cast<int>((n + 255) / 256);
     if (blocks > kBBoxBlocks) blocks = kBBoxBlocks;
     if (blocks < 1) blocks = 1;
-    bbox_kernel<<<blocks, 256, 0, st>>>(pos, n, w.bbox_partial, w.bbox_counter, w.box);
+    launch_behind(bbox_kernel, dim3(blocks), dim3(256), 0, st, pos, n, w.bbox_partial, w.bbox_counter, w.box);
     if (timer) timer->end(kStageBBox, st);
     return cudaGetLastError();
 }
@@ -1395,9 +1411,11 @@ cudaError_t bh_bbox(const float4 *pos, int64_t n, BHWorkspace &w, cudaStream_t s
 cudaError_t bh_keys(const float4 *pos, int64_t n, BHWorkspace &w, int mode, cudaStream_t st, StageTimer *timer) {
     if (timer) timer->begin(kStageMorton, st);
     if (mode == NBODY_KEYS_MORTON)
-        morton_kernel<NBODY_KEYS_MORTON><<<grid_for(n, 256), 256, 0, st>>>(pos, n, w.box, w.keys[0], w.vals[0]);
+        launch_behind(morton_kernel<NBODY_KEYS_MORTON>, dim3(grid_for(n, 256)), dim3(256), 0, st, pos, n, w.box,
+                      w.keys[0], w.vals[0]);
     else
-        morton_kernel<NBODY_KEYS_OCTREE><<<grid_for(n, 256), 256, 0, st>>>(pos, n, w.box, w.keys[0], w.vals[0]);
+        launch_behind(morton_kernel<NBODY_KEYS_OCTREE>, dim3(grid_for(n, 256)), dim3(256), 0, st, pos, n, w.box,
+                      w.keys[0], w.vals[0]);
     if (timer) timer->end(kStageMorton, st);
     return cudaGetLastError();
 }
@@ -1419,8 +1437,8 @@ cudaError_t bh_gather(int64_t n, const BHWorkspace &w, const float4 *pos_in, con
                       const float4 *acc_in, const int *id_in, float4 *pos_out, float4 *vel_out, float4 *acc_out,
                       int *id_out, cudaStream_t st, int *status, StageTimer *timer) {
     if (timer) timer->begin(kStageGather, st);
-    gather_kernel<<<grid_for(n, 256), 256, 0, st>>>(w.vals[0], n, pos_in, vel_in, acc_in, id_in, pos_out, vel_out,
-                                                    acc_out, id_out, status, nullptr, nullptr, w.mask);
+    launch_behind(gather_kernel, dim3(grid_for(n, 256)), dim3(256), 0, st, w.vals[0], n, pos_in, vel_in, acc_in,
+                  id_in, pos_out, vel_out, acc_out, id_out, status, nullptr, nullptr, w.mask);
     if (timer) timer->end(kStageGather, st);
     return cudaGetLastError();
 }
@@ -1447,33 +1465,35 @@ cudaError_t bh_build(const float4 *pos_sorted, int64_t n, BHWorkspace &w, cudaSt
     // Records: at most 2n (n - 1 cells and n leaves).
     const int64_t cap = 2 * (n > 1 ? n : 2);
     const int tiles = static_cast<int>((n + kScanTile - 1) / kScanTile);
-    radix_tree_kernel<<<grid_for(n, 256), 256, 0, st>>>(k, n, w.tree, sv, w.mask, sv.seg ? 32 : 0, w.scan_words, tiles + 1,
-                                                        reinterpret_cast<int4 *>(w.kids),
-                                                        levels ? nullptr : w.rec.arrive);
-    count_scan_kernel<<<tiles, kScanThreads, 0, st>>>(k, n, w.mask, sv, w.P, w.scan_words, status);
-    emit_kernel<<<grid_for(n, 256), 256, 0, st>>>(k, n, pos_sorted, w.tree, w.mask, w.P, w.box, w.nodes, w.rec, w.kids, sv,
-                                                  !levels);
+    launch_behind(radix_tree_kernel, dim3(grid_for(n, 256)), dim3(256), 0, st, k, n, w.tree, sv, w.mask,
+                  sv.seg ? 32 : 0, w.scan_words, tiles + 1, reinterpret_cast<int4 *>(w.kids),
+                  levels ? nullptr : w.rec.arrive);
+    launch_behind(count_scan_kernel, dim3(tiles), dim3(kScanThreads), 0, st, k, n, w.mask, sv, w.P, w.scan_words,
+                  status);
+    launch_behind(emit_kernel, dim3(grid_for(n, 256)), dim3(256), 0, st, k, n, pos_sorted, w.tree, w.mask, w.P,
+                  w.box, w.nodes, w.rec, w.kids, sv, !levels);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     if (timer) timer->end(kStageBuild, st);
     if (timer) timer->begin(kStageUpsweep, st);
     if (!levels) {
-        upsweep_climb_kernel<<<grid_for(n, 256), 256, 0, st>>>(k, n, pos_sorted, w.mask, w.P, w.nodes, w.rec,
-                                                               w.kids, father_depth(n), status, sv);
+        launch_behind(upsweep_climb_kernel, dim3(grid_for(n, 256)), dim3(256), 0, st, k, n, pos_sorted, w.mask, w.P,
+                      w.nodes, w.rec, w.kids, father_depth(n), status, sv);
         if (timer) timer->end(kStageUpsweep, st);
         return cudaGetLastError();
     }
     e = cudaMemsetAsync(w.rec.lvl, 0, sizeof(unsigned) * 96, st);
     if (e != cudaSuccess) return e;
-    bucket_cm_kernel<<<grid_for(n, 256), 256, 0, st>>>(k, n, pos_sorted, w.mask, w.P, w.nodes, sv);
+    launch_behind(bucket_cm_kernel, dim3(grid_for(n, 256)), dim3(256), 0, st, k, n, pos_sorted, w.mask, w.P, w.nodes,
+                  sv);
     const unsigned spread = static_cast<unsigned>(std::min<int64_t>(grid_for(n, 256), 1216));
-    level_count_kernel<<<spread, 256, 0, st>>>(w.rec.level, w.P + n, w.rec.lvl);
-    level_scatter_kernel<<<grid_for(cap, 256), 256, 0, st>>>(w.rec.level, w.P + n, w.rec.lvl, w.rec.list, cap,
-                                                             status);
+    launch_behind(level_count_kernel, dim3(spread), dim3(256), 0, st, w.rec.level, w.P + n, w.rec.lvl);
+    launch_behind(level_scatter_kernel, dim3(grid_for(cap, 256)), dim3(256), 0, st, w.rec.level, w.P + n, w.rec.lvl,
+                  w.rec.list, cap, status);
     const int fd = father_depth(n);
     for (int L = kMaxLevel - 1; L >= 0; --L)
-        level_cm_kernel<<<spread, 256, 0, st>>>(L, w.nodes, w.rec.level, w.kids, w.rec.list, w.rec.lvl, fd,
-                                                sv);
+        launch_behind(level_cm_kernel, dim3(spread), dim3(256), 0, st, L, w.nodes, w.rec.level, w.kids, w.rec.list,
+                      w.rec.lvl, fd, sv);
     if (timer) timer->end(kStageUpsweep, st);
     return cudaGetLastError();
 }
@@ -1488,17 +1508,16 @@ void launch_walk(const BHWorkspace &w, unsigned blocks, cudaStream_t st, const u
                  const HostOut &host = HostOut{}) {
     if constexpr (!SEG && !POT) {
         if (w.walk == kWalkCell && host.pos) {
-            cell_walk_kernel<COUNT, POT, SEG, GUARD, true><<<blocks * 4, 64, 0, st>>>(
-                w.nodes, w.kids, node_total, pos, n, eps2, theta2, dt, pos_out, vel, acc, force_out, ids, counters,
-                phi_out, euler, work, nwork, params, P, host);
+            launch_behind(cell_walk_kernel<COUNT, POT, SEG, GUARD, true>, dim3(blocks * 4), dim3(64), 0, st, w.nodes,
+                          w.kids, node_total, pos, n, eps2, theta2, dt, pos_out, vel, acc, force_out, ids, counters,
+                          phi_out, euler, work, nwork, params, P, host);
             return;
         }
     }
     if (w.walk == kWalkCell)
-        cell_walk_kernel<COUNT, POT, SEG, GUARD><<<blocks * 4, 64, 0, st>>>(w.nodes, w.kids, node_total,
-                                                                         pos, n, eps2, theta2, dt, pos_out, vel, acc, force_out,
-                                                                         ids, counters, phi_out, euler, work, nwork,
-                                                                         params, P, host);
+        launch_behind(cell_walk_kernel<COUNT, POT, SEG, GUARD>, dim3(blocks * 4), dim3(64), 0, st, w.nodes, w.kids,
+                      node_total, pos, n, eps2, theta2, dt, pos_out, vel, acc, force_out, ids, counters, phi_out,
+                      euler, work, nwork, params, P, host);
     else
         traverse2_kernel<COUNT, POT, SEG, GUARD><<<blocks, 256, 0, st>>>(w.nodes, node_total, pos, n, eps2, theta2,
                                                                          dt, pos_out, vel, acc, force_out, ids,
@@ -1591,15 +1610,15 @@ cudaError_t bh_ensemble_step(int64_t n, BHWorkspace &w, const BHEnsembleTables &
     if (n <= 0 || e.systems <= 0) return cudaSuccess;
     cudaError_t err;
     if (tm) tm->begin(kStageBBox, st);
-    bbox_seg_kernel<<<e.nchunks, 256, 0, st>>>(P, e.chunks, e.box_acc, e.boxes);
+    launch_behind(bbox_seg_kernel, dim3(e.nchunks), dim3(256), 0, st, P, e.chunks, e.box_acc, e.boxes);
     if (tm) tm->end(kStageBBox, st);
     if (tm) tm->begin(kStageMorton, st);
     if (key_mode == NBODY_KEYS_MORTON)
-        keys_seg_kernel<NBODY_KEYS_MORTON><<<grid_for(n, 256), 256, 0, st>>>(P, n, e.seg, e.boxes, w.keys[0],
-                                                                              e.keys_orig, w.vals[0]);
+        launch_behind(keys_seg_kernel<NBODY_KEYS_MORTON>, dim3(grid_for(n, 256)), dim3(256), 0, st, P, n, e.seg,
+                      e.boxes, w.keys[0], e.keys_orig, w.vals[0]);
     else
-        keys_seg_kernel<NBODY_KEYS_OCTREE><<<grid_for(n, 256), 256, 0, st>>>(P, n, e.seg, e.boxes, w.keys[0],
-                                                                              e.keys_orig, w.vals[0]);
+        launch_behind(keys_seg_kernel<NBODY_KEYS_OCTREE>, dim3(grid_for(n, 256)), dim3(256), 0, st, P, n, e.seg,
+                      e.boxes, w.keys[0], e.keys_orig, w.vals[0]);
     if (tm) tm->end(kStageMorton, st);
     if (tm) tm->begin(kStageSort, st);
     // Stable by key over all systems, then stable by system: within each
@@ -1610,7 +1629,7 @@ cudaError_t bh_ensemble_step(int64_t n, BHWorkspace &w, const BHEnsembleTables &
     uint64_t *k0 = alt ? w.keys[1] : w.keys[0], *k1 = alt ? w.keys[0] : w.keys[1];
     uint32_t *v0 = alt ? w.vals[1] : w.vals[0], *v1 = alt ? w.vals[0] : w.vals[1];
     if (e.systems > 1) {
-        seg_keys_kernel<<<grid_for(n, 256), 256, 0, st>>>(v0, n, e.seg, k0, status);
+        launch_behind(seg_keys_kernel, dim3(grid_for(n, 256)), dim3(256), 0, st, v0, n, e.seg, k0, status);
         err = sort_pairs(k0, v0, k1, v1, n, w.sort_scratch, st, status, &alt, e.seg_passes);
         if (err != cudaSuccess) return err;
         if (alt) {
@@ -1621,8 +1640,8 @@ cudaError_t bh_ensemble_step(int64_t n, BHWorkspace &w, const BHEnsembleTables &
     if (tm) tm->begin(kStageGather, st);
     // Sorted keys into keys[0] (the build reads them there), permutation in vals[0].
     uint64_t *ksorted = w.keys[0];
-    gather_kernel<<<grid_for(n, 256), 256, 0, st>>>(v0, n, P, V, A, I, Po, Vo, Ao, Io, status, e.keys_orig, ksorted,
-                                                    w.mask);
+    launch_behind(gather_kernel, dim3(grid_for(n, 256)), dim3(256), 0, st, v0, n, P, V, A, I, Po, Vo, Ao, Io, status,
+                  e.keys_orig, ksorted, w.mask);
     if (tm) tm->end(kStageGather, st);
     err = cudaGetLastError();
     if (err != cudaSuccess) return err;

@@ -97,6 +97,11 @@ __device__ __forceinline__ void tma_bulk_g2s(void *dst_smem, const void *src_gme
         : "memory");
 }
 
+// Waits until the kernels that this one was launched behind (launch_behind)
+// have completed and their writes are visible; returns at once in a kernel
+// launched otherwise. Every access to memory they touch comes after it.
+__device__ __forceinline__ void wait_for_launches_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // 1/sqrt(x), hardware approximation, flush-to-zero (inputs here are >= eps^2).
 __device__ __forceinline__ float rsqrt_ftz(float x) {
     float y;

@@ -42,6 +42,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "launch.h"
 #include "pp_common.cuh"
 
 namespace nbody {
@@ -324,7 +325,7 @@ __global__ void __launch_bounds__(kSymT) pp_sym_sum_kernel(const float4 *__restr
                                                            const float *__restrict__ rows,
                                                            Integrate g) {
     constexpr int kBatch = 16;
-    asm volatile("griddepcontrol.wait;" ::: "memory");  // the parts and rows are written
+    wait_for_launches_before();
     const int to = blockIdx.x / (kSymB / kSymT), i0 = (blockIdx.x % (kSymB / kSymT)) * kSymT + threadIdx.x;
     const int64_t i = static_cast<int64_t>(to) * kSymB + i0;
     if (i >= n) return;
@@ -443,18 +444,8 @@ cudaError_t pp_sym_launch(const SymPlan &p, const float4 *pos, int64_t n, float 
         pp_sym_kernel<true><<<p.ctas, kSymT, 0, stream>>>(pos, n, eps2, p, parts, rows, status);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    // Launched while the last CTAs of the sums run (it waits for them itself).
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(static_cast<unsigned>((n + kSymT - 1) / kSymT));
-    cfg.blockDim = dim3(kSymT);
-    cfg.stream = stream;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, pp_sym_sum_kernel, pos, n, p, static_cast<const float *>(parts),
-                              static_cast<const float *>(rows), g);
+    return launch_behind(pp_sym_sum_kernel, dim3(static_cast<unsigned>((n + kSymT - 1) / kSymT)), dim3(kSymT), 0, stream, pos,
+                         n, p, parts, rows, g);
 }
 
 }  // namespace nbody

@@ -17,6 +17,7 @@
 #include <cuda_runtime.h>
 
 #include "common.cuh"
+#include "launch.h"
 #include "sort.h"
 
 namespace nbody {
@@ -75,6 +76,7 @@ __global__ void __launch_bounds__(T) block_sort_kernel(const uint64_t *keys_in, 
     uint64_t *k = reinterpret_cast<uint64_t *>(smem);
     uint32_t *v = reinterpret_cast<uint32_t *>(k + padded(kTile));
     const int tid = threadIdx.x;
+    wait_for_launches_before();
     const int64_t base = static_cast<int64_t>(blockIdx.x) * kTile;
     const int count = n - base < kTile ? static_cast<int>(n - base) : kTile;
 #pragma unroll
@@ -167,7 +169,7 @@ __global__ void __launch_bounds__(kMergeThreads) merge_pass_kernel(const uint64_
     __shared__ uint32_t v[padded(kMergeOut)];
     __shared__ int64_t split[2];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    asm volatile("griddepcontrol.wait;" ::: "memory");  // the runs are written
+    wait_for_launches_before();
     const int64_t o0 = static_cast<int64_t>(blockIdx.x) * kMergeOut;  // 2 * run is a multiple of kMergeOut
     const int64_t pair = o0 / (2 * run) * (2 * run);
     const int64_t la = n - pair < run ? n - pair : run;
@@ -248,24 +250,13 @@ cudaError_t merge_sort_pairs(uint64_t *keys, uint32_t *vals, uint64_t *keys_alt,
     uint64_t *ki = passes % 2 ? keys_alt : keys, *ko = passes % 2 ? keys : keys_alt;
     uint32_t *vi = passes % 2 ? vals_alt : vals, *vo = passes % 2 ? vals : vals_alt;
     const unsigned blocks = static_cast<unsigned>((n + tile - 1) / tile);
-    if (tile == 2048)
-        block_sort_kernel<512, 4><<<blocks, 512, block_smem<512, 4>(), stream>>>(keys, vals, ki, vi, n);
-    else
-        block_sort_kernel<512, 8><<<blocks, 512, block_smem<512, 8>(), stream>>>(keys, vals, ki, vi, n);
-    cudaError_t e = cudaGetLastError();
-    // Each pass is launched while the one before drains (and waits for it itself).
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(static_cast<unsigned>((n + kMergeOut - 1) / kMergeOut));
-    cfg.blockDim = dim3(kMergeThreads);
-    cfg.stream = stream;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cudaError_t e = tile == 2048 ? launch_behind(block_sort_kernel<512, 4>, dim3(blocks), dim3(512), block_smem<512, 4>(),
+                                                 stream, keys, vals, ki, vi, n)
+                                 : launch_behind(block_sort_kernel<512, 8>, dim3(blocks), dim3(512), block_smem<512, 8>(),
+                                                 stream, keys, vals, ki, vi, n);
     for (int64_t run = tile; run < n && e == cudaSuccess; run *= 2) {
-        e = cudaLaunchKernelEx(&cfg, merge_pass_kernel, static_cast<const uint64_t *>(ki), static_cast<const uint32_t *>(vi),
-                               ko, vo, n, run);
+        e = launch_behind(merge_pass_kernel, dim3(static_cast<unsigned>((n + kMergeOut - 1) / kMergeOut)),
+                          dim3(kMergeThreads), 0, stream, ki, vi, ko, vo, n, run);
         uint64_t *tk = ki; ki = ko; ko = tk;
         uint32_t *tv = vi; vi = vo; vo = tv;
     }

@@ -31,6 +31,7 @@
 #include "bh.h"
 #include "bh_walk.cuh"
 #include "common.cuh"
+#include "launch.h"
 
 namespace nbody {
 
@@ -115,6 +116,7 @@ __global__ void __launch_bounds__(32 * W, W >= 16 && !SEG ? 1 : 32 / W) team_wal
     const float4 *__restrict__ params, const uint32_t *__restrict__ P, const HostOut host) {
     __shared__ __align__(16) TeamArea<W> A;
     constexpr int S = TeamArea<W>::S;
+    wait_for_launches_before();
     unsigned long long n_pairs = 0, n_visits = 0;
     float phi = 0.f;  // no potential in this form
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -349,33 +351,23 @@ __global__ void __launch_bounds__(32 * W, W >= 16 && !SEG ? 1 : 32 / W) team_wal
 }
 
 template <int W, bool COUNT, bool SEG, bool GUARD>
-void launch_form(const TeamWalk &a, unsigned sets, cudaStream_t st) {
-    if constexpr (!SEG) {
-        if (a.host.pos) {
-            team_walk_kernel<W, COUNT, SEG, GUARD, true><<<sets, 32 * W, 0, st>>>(
-                a.nodes, a.kids, a.node_total, a.pos, a.n, a.eps2, a.theta2, a.dt, a.pos_out, a.vel, a.acc, a.force_out,
-                a.ids, a.counters, a.euler, a.work, a.params, a.P, a.host);
-            return;
-        }
-    }
-    team_walk_kernel<W, COUNT, SEG, GUARD, false><<<sets, 32 * W, 0, st>>>(
-        a.nodes, a.kids, a.node_total, a.pos, a.n, a.eps2, a.theta2, a.dt, a.pos_out, a.vel, a.acc, a.force_out, a.ids,
-        a.counters, a.euler, a.work, a.params, a.P, a.host);
+cudaError_t launch_form(const TeamWalk &a, unsigned sets, cudaStream_t st) {
+    const auto launch = [&](auto kernel) {
+        return launch_behind(kernel, dim3(sets), dim3(32 * W), 0, st, a.nodes, a.kids, a.node_total, a.pos, a.n, a.eps2,
+                             a.theta2, a.dt, a.pos_out, a.vel, a.acc, a.force_out, a.ids, a.counters, a.euler, a.work,
+                             a.params, a.P, a.host);
+    };
+    if constexpr (!SEG)
+        if (a.host.pos) return launch(team_walk_kernel<W, COUNT, SEG, GUARD, true>);
+    return launch(team_walk_kernel<W, COUNT, SEG, GUARD, false>);
 }
 
 template <int W>
-void launch_team(const TeamWalk &a, bool guard, unsigned sets, cudaStream_t st) {
+cudaError_t launch_team(const TeamWalk &a, bool guard, unsigned sets, cudaStream_t st) {
     const bool seg = a.work != nullptr;
-    if (a.counters) {
-        if (seg) launch_form<W, true, true, true>(a, sets, st);
-        else launch_form<W, true, false, true>(a, sets, st);
-    } else if (seg) {
-        if (guard) launch_form<W, false, true, true>(a, sets, st);
-        else launch_form<W, false, true, false>(a, sets, st);
-    } else {
-        if (guard) launch_form<W, false, false, true>(a, sets, st);
-        else launch_form<W, false, false, false>(a, sets, st);
-    }
+    if (a.counters) return seg ? launch_form<W, true, true, true>(a, sets, st) : launch_form<W, true, false, true>(a, sets, st);
+    if (seg) return guard ? launch_form<W, false, true, true>(a, sets, st) : launch_form<W, false, true, false>(a, sets, st);
+    return guard ? launch_form<W, false, false, true>(a, sets, st) : launch_form<W, false, false, false>(a, sets, st);
 }
 
 }  // namespace
@@ -406,13 +398,12 @@ cudaError_t bh_team_walk(const TeamWalk &a, int team, bool guard, int64_t sets, 
     if (sets <= 0) return cudaSuccess;
     const unsigned g = static_cast<unsigned>(sets);
     switch (team) {
-        case 2: launch_team<2>(a, guard, g, st); break;
-        case 4: launch_team<4>(a, guard, g, st); break;
-        case 8: launch_team<8>(a, guard, g, st); break;
-        case 16: launch_team<16>(a, guard, g, st); break;
+        case 2: return launch_team<2>(a, guard, g, st);
+        case 4: return launch_team<4>(a, guard, g, st);
+        case 8: return launch_team<8>(a, guard, g, st);
+        case 16: return launch_team<16>(a, guard, g, st);
         default: return cudaErrorInvalidValue;
     }
-    return cudaGetLastError();
 }
 
 }  // namespace nbody

@@ -6,14 +6,16 @@
 // block scan, look-back, scatter): 105 us for 4,096 pairs and 121 us for
 // 65,536. Here a CTA sorts a tile in shared memory in one launch (four or
 // eight pairs per thread in registers, then merge rounds over twice as many
-// threads each), and each further launch merges neighbouring runs in pairs,
-// every CTA producing 2,048 pairs from the part of two runs that a search along
-// the merge path gives it. Taking the left run first where keys are equal keeps
-// the sort stable, so the permutation is the radix sort's. GB300, us, radix /
-// merge: 4,096 pairs 105 / 19, 30,001 120 / 40, 65,536 121 / 47, 262,144 137 /
-// 63, 2^20 212 / 124, 2^22 553 / 452. A tile takes 14 us (2,048 pairs), a merge pass
-// 7 us while the launches and the chain of its searches bound it (up to 2^18
-// pairs), 12 us of traffic at 2^20.
+// threads each), and each further launch merges neighbouring runs: four or eight
+// at a time by searching every pair's place (rank_merge_kernel) up to 2^18 pairs,
+// two at a time above, every CTA producing 2,048 pairs from the part of two runs
+// that a search along the merge path gives it (merge_pass_kernel). Taking the
+// left run first where keys are equal keeps the sort stable, so the permutation
+// is the radix sort's. GB300, us, radix / merge: 4,096 pairs 105 / 17, 30,001
+// 120 / 22, 65,536 121 / 26, 262,144 137 / 53, 2^20 212 / 121, 2^22 553 / 452.
+// A tile of 2,048 pairs takes 10 us, a pass by searching 5 us up to 2^17 pairs, a
+// merge pass 7 us while its launch and the chain of its searches bound it and
+// 12 us of traffic at 2^20.
 #include <cuda_runtime.h>
 
 #include "common.cuh"
@@ -27,6 +29,9 @@ namespace {
 constexpr int kMergeThreads = 256;
 constexpr int kMergeItems = 8;
 constexpr int kMergeOut = kMergeThreads * kMergeItems;  // pairs per CTA of a merge pass
+
+constexpr int kRankThreads = 128;
+constexpr int kRankSearches = 4;
 
 // Places in shared memory: one left free in every 16, so that threads whose
 // items lie side by side do not meet in the banks.
@@ -217,6 +222,54 @@ __global__ void __launch_bounds__(kMergeThreads) merge_pass_kernel(const uint64_
     }
 }
 
+// Groups of `ways` runs (four or eight) of 2^run_bits pairs, the last ones
+// shorter or missing, into one run each: a pair's place is its own place in its
+// run plus what a binary search finds before it in each other run of its group
+// (its equals in earlier runs included, those in later ones not: stable).
+// A step of a search waits for a load, so four searches go side by side. The
+// group's size is left to run time: with four or eight as a constant the same
+// loop took 30 instead of 22 us for 30,001 pairs (sort of all tiles included).
+__global__ void __launch_bounds__(kRankThreads) rank_merge_kernel(const uint64_t *__restrict__ keys_in,
+                                                                  const uint32_t *__restrict__ vals_in,
+                                                                  uint64_t *__restrict__ keys_out,
+                                                                  uint32_t *__restrict__ vals_out, int n, int run_bits,
+                                                                  int ways) {
+    wait_for_launches_before();
+    const int i = blockIdx.x * kRankThreads + threadIdx.x;
+    if (i >= n) return;
+    const int run = 1 << run_bits, mine = i >> run_bits, first = mine & ~(ways - 1);
+    const uint64_t x = keys_in[i];
+    const uint32_t v = vals_in[i];
+    int to = i - (mine - first) * run;
+    for (int s0 = 0; s0 < ways; s0 += kRankSearches) {
+        int at[kRankSearches], end[kRankSearches];
+        uint64_t bound[kRankSearches];  // the keys below it come first
+#pragma unroll
+        for (int j = 0; j < kRankSearches; ++j) {
+            const int s = first + s0 + j;
+            const bool other = s != mine && s * run < n;
+            at[j] = other ? s * run : 0;
+            end[j] = other ? (n - at[j] < run ? n : at[j] + run) : 0;
+            to -= at[j];
+            bound[j] = x;
+            if (s < mine) {
+                if (x == ~0ull) at[j] = end[j]; else bound[j] = x + 1;
+            }
+        }
+        for (int step = run; step > 0; step >>= 1) {
+            uint64_t k[kRankSearches];
+#pragma unroll
+            for (int j = 0; j < kRankSearches; ++j) k[j] = keys_in[at[j] + step <= end[j] ? at[j] + step - 1 : 0];
+#pragma unroll
+            for (int j = 0; j < kRankSearches; ++j) at[j] += at[j] + step <= end[j] && k[j] < bound[j] ? step : 0;
+        }
+#pragma unroll
+        for (int j = 0; j < kRankSearches; ++j) to += at[j];
+    }
+    keys_out[to] = x;
+    vals_out[to] = v;
+}
+
 template <int T, int N>
 constexpr size_t block_smem() {
     return static_cast<size_t>(padded(T * N)) * (sizeof(uint64_t) + sizeof(uint32_t));
@@ -229,10 +282,22 @@ cudaError_t prepare_block() {
 }
 
 // Tiles of 2,048 pairs while passes are cheaper than the larger tile's rounds
-// (262,144 pairs: 62.6 us against 65.7 with 4,096 and 76.5 with 8,192 per tile;
-// 524,288: 86 / 80 / 90).
+// (262,144 pairs: 53 us against 60 with 4,096 per tile; 524,288, merging in
+// pairs: 86 with 2,048, 80 with 4,096, 90 with 8,192).
 constexpr int64_t kSmallTiles = 1 << 18;
 int64_t tile_of(int64_t n) { return n <= kSmallTiles ? 2048 : 4096; }
+
+// Runs merged by the next pass over runs of `run` pairs. Up to 2^18 pairs a pass
+// is bound by its launch and a chain of loads, not by traffic, and places found
+// by searching merge four or eight runs in about the time of one pass of two:
+// whole sorts of 8,192 / 30,001 / 65,536 / 131,072 / 262,144 pairs take 16.6 /
+// 21.7 / 25.5 / 30.1 / 53.4 us against 23.6 / 37.9 / 45.0 / 52.8 / 61.0 in
+// pairs; above, the searches' loads cost more (524,288: 97 against 77 us).
+// Eight at once only for the last pass (16,384: 18.7 against 22.4 us by fours).
+int merge_ways(int64_t n, int64_t run) {
+    if (n > kSmallTiles) return 2;
+    return n > 4 * run && n <= 8 * run ? 8 : 4;
+}
 
 }  // namespace
 
@@ -244,8 +309,7 @@ cudaError_t merge_sort_prepare() {
 cudaError_t merge_sort_pairs(uint64_t *keys, uint32_t *vals, uint64_t *keys_alt, uint32_t *vals_alt, int64_t n,
                              cudaStream_t stream) {
     const int64_t tile = tile_of(n);
-    int passes = 0;
-    for (int64_t run = tile; run < n; run *= 2) ++passes;
+    const int passes = merge_sort_launches(n) - 1;
     // A tile may be sorted in place; the last pass ends in keys.
     uint64_t *ki = passes % 2 ? keys_alt : keys, *ko = passes % 2 ? keys : keys_alt;
     uint32_t *vi = passes % 2 ? vals_alt : vals, *vo = passes % 2 ? vals : vals_alt;
@@ -254,9 +318,19 @@ cudaError_t merge_sort_pairs(uint64_t *keys, uint32_t *vals, uint64_t *keys_alt,
                                                  stream, keys, vals, ki, vi, n)
                                  : launch_behind(block_sort_kernel<512, 8>, dim3(blocks), dim3(512), block_smem<512, 8>(),
                                                  stream, keys, vals, ki, vi, n);
-    for (int64_t run = tile; run < n && e == cudaSuccess; run *= 2) {
-        e = launch_behind(merge_pass_kernel, dim3(static_cast<unsigned>((n + kMergeOut - 1) / kMergeOut)),
-                          dim3(kMergeThreads), 0, stream, ki, vi, ko, vo, n, run);
+    for (int64_t run = tile; run < n && e == cudaSuccess;) {
+        const int ways = merge_ways(n, run);
+        if (ways == 2) {
+            e = launch_behind(merge_pass_kernel, dim3(static_cast<unsigned>((n + kMergeOut - 1) / kMergeOut)),
+                              dim3(kMergeThreads), 0, stream, ki, vi, ko, vo, n, run);
+        } else {
+            int bits = 0;
+            while ((int64_t(1) << bits) < run) ++bits;
+            e = launch_behind(rank_merge_kernel,
+                              dim3(static_cast<unsigned>((n + kRankThreads - 1) / kRankThreads)), dim3(kRankThreads), 0,
+                              stream, ki, vi, ko, vo, static_cast<int>(n), bits, ways);
+        }
+        run *= ways;
         uint64_t *tk = ki; ki = ko; ko = tk;
         uint32_t *tv = vi; vi = vo; vo = tv;
     }
@@ -265,7 +339,7 @@ cudaError_t merge_sort_pairs(uint64_t *keys, uint32_t *vals, uint64_t *keys_alt,
 
 int merge_sort_launches(int64_t n) {
     int launches = 1;
-    for (int64_t run = tile_of(n); run < n; run *= 2) ++launches;
+    for (int64_t run = tile_of(n); run < n; run *= merge_ways(n, run)) ++launches;
     return launches;
 }
 

@@ -42,3 +42,9 @@ def test_sort_forms_are_stable(nb, cuda, monkeypatch, form, n):
         np.testing.assert_array_equal(k.cpu().numpy().view(np.uint64), keys[order])
         np.testing.assert_array_equal(v.cpu().numpy().view(np.uint32), vals[order])
     solver.close()
+
+
+@pytest.mark.parametrize("n", [4096, 6145, 8192, 14337, 16384, 16385, 32768, 32769, 65537, 131073, 262143])
+def test_sort_by_searched_places(nb, cuda, monkeypatch, n):
+    """Groups of four and of eight runs, whole and cut short, in one to three passes."""
+    test_sort_forms_are_stable(nb, cuda, monkeypatch, "merge", n)

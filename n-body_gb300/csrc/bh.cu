@@ -1060,8 +1060,9 @@ __global__ void __launch_bounds__(64, (COUNT || SEG) ? 16 : 24) cell_walk_kernel
     const float4 *__restrict__ pos, int64_t n, float eps2, float theta2, float dt, float4 *__restrict__ pos_out,
     float4 *__restrict__ vel, float4 *__restrict__ acc, float4 *__restrict__ force_out, const int *__restrict__ ids,
     unsigned long long *__restrict__ counters, float *__restrict__ phi_out, int euler, const int4 *__restrict__ work,
-    int nwork, const float4 *__restrict__ params, const uint32_t *__restrict__ P, const HostOut host) {
+    int nwork, const float4 *__restrict__ params, const uint32_t *__restrict__ P, const HostOut host, int beside) {
     wait_for_launches_before();
+    if (beside & kWalkLetsNext) let_next_launch_begin();
     // One block of shared memory per warp, addressed from one base.
     struct __align__(16) WarpArea {
         int4 stk_i[kCellDepth];     // cell, mask A, mask B, box hz (float bits)
@@ -1505,19 +1506,19 @@ void launch_walk(const BHWorkspace &w, unsigned blocks, cudaStream_t st, const u
                  const float4 *pos, int64_t n, float eps2, float theta2, float dt, float4 *pos_out, float4 *vel,
                  float4 *acc, float4 *force_out, const int *ids, unsigned long long *counters, float *phi_out,
                  int euler, const int4 *work, int nwork, const float4 *params, const uint32_t *P,
-                 const HostOut &host = HostOut{}) {
+                 const HostOut &host = HostOut{}, int beside = 0) {
     if constexpr (!SEG && !POT) {
         if (w.walk == kWalkCell && host.pos) {
             launch_behind(cell_walk_kernel<COUNT, POT, SEG, GUARD, true>, dim3(blocks * 4), dim3(64), 0, st, w.nodes,
                           w.kids, node_total, pos, n, eps2, theta2, dt, pos_out, vel, acc, force_out, ids, counters,
-                          phi_out, euler, work, nwork, params, P, host);
+                          phi_out, euler, work, nwork, params, P, host, beside);
             return;
         }
     }
     if (w.walk == kWalkCell)
         launch_behind(cell_walk_kernel<COUNT, POT, SEG, GUARD>, dim3(blocks * 4), dim3(64), 0, st, w.nodes, w.kids,
                       node_total, pos, n, eps2, theta2, dt, pos_out, vel, acc, force_out, ids, counters, phi_out,
-                      euler, work, nwork, params, P, host);
+                      euler, work, nwork, params, P, host, beside);
     else
         traverse2_kernel<COUNT, POT, SEG, GUARD><<<blocks, 256, 0, st>>>(w.nodes, node_total, pos, n, eps2, theta2,
                                                                          dt, pos_out, vel, acc, force_out, ids,
@@ -1543,8 +1544,11 @@ cudaError_t bh_traverse(const float4 *pos_sorted, int64_t n, const BHWorkspace &
     if (host.pos && !bh_walk_writes_host(w)) return cudaErrorInvalidValue;
     if (timer) timer->begin(kStageTraverse, st);
     // The record count P[n] stays on the device; the kernel reads it.
-    const int team = bh_walk_team(w, n);
-    if (team > 1) {
+    if (w.bodies_per_lane == 2) {
+        const bool cell = w.walk == kWalkCell, guard = !(eps2 > 0.f && theta2 > 0.f);
+        const int team = bh_walk_team(w, n);
+        const int64_t sets = (n + 63) / 64, main = cell ? bh_main_sets(n) : sets;
+        const int beside = main < sets ? kWalkLetsNext : 0;
         TeamWalk a;
         a.nodes = w.nodes;
         a.kids = w.kids;
@@ -1562,23 +1566,29 @@ cudaError_t bh_traverse(const float4 *pos_sorted, int64_t n, const BHWorkspace &
         a.counters = w.counters;
         a.euler = euler;
         a.host = host;
-        const cudaError_t e = bh_team_walk(a, team, !(eps2 > 0.f && theta2 > 0.f), (n + 63) / 64, st);
-        if (e != cudaSuccess) return e;
-    } else if (w.bodies_per_lane == 2) {
-        const int64_t warps = (n + 63) / 64;
-        const unsigned blocks = static_cast<unsigned>((warps * 32 + 255) / 256);
-        if (w.counters)
+        a.beside = beside;
+        cudaError_t e = cudaSuccess;
+        const unsigned blocks = static_cast<unsigned>((main * 32 + 255) / 256);
+        if (team > 1)
+            e = bh_team_walk(a, team, guard, main, st);
+        else if (w.counters)
             launch_walk<true, false, false, true>(w, blocks, st, w.P + n, pos_sorted, n, eps2, theta2, dt, pos_out, vel,
                                                  acc, force_out, ids, w.counters, nullptr, euler, nullptr, 0, nullptr,
-                                                 nullptr, host);
-        else if (eps2 > 0.f && theta2 > 0.f)
+                                                 nullptr, host, beside);
+        else if (!guard)
             launch_walk<false, false, false, false>(w, blocks, st, w.P + n, pos_sorted, n, eps2, theta2, dt, pos_out,
                                                    vel, acc, force_out, ids, nullptr, nullptr, euler, nullptr, 0,
-                                                   nullptr, nullptr, host);
+                                                   nullptr, nullptr, host, beside);
         else
             launch_walk<false, false, false, true>(w, blocks, st, w.P + n, pos_sorted, n, eps2, theta2, dt, pos_out,
                                                   vel, acc, force_out, ids, nullptr, nullptr, euler, nullptr, 0,
-                                                  nullptr, nullptr, host);
+                                                  nullptr, nullptr, host, beside);
+        if (e == cudaSuccess && main < sets) {
+            a.first = main;
+            a.beside = kWalkWaitsLast;
+            e = bh_team_walk(a, kTailTeam, guard, sets - main, st);
+        }
+        if (e != cudaSuccess) return e;
     } else if (w.counters)
         traverse_kernel<true><<<grid_for(n, 256), 256, 0, st>>>(w.nodes, w.P + n, pos_sorted, n, eps2, theta2, dt,
                                                                 pos_out, vel, acc, force_out, ids, w.counters, euler);
@@ -1652,11 +1662,15 @@ cudaError_t bh_ensemble_step(int64_t n, BHWorkspace &w, const BHEnsembleTables &
     err = bh_build(Po, n, w, st, status, tm, sv);
     if (err != cudaSuccess) return err;
     if (tm) tm->begin(kStageTraverse, st);
-    // One launch per run of systems with the same team size.
+    // One launch per team size, side by side.
     const int4 *work = e.warps;
-    for (const std::pair<int, int> &run : e.teams) {
-        const int team = w.walk == kWalkCell ? run.first : 1;
-        const int sets = run.second;
+    const size_t runs = e.teams.size();
+    for (size_t r = 0; r < runs; ++r) {
+        const bool cell = w.walk == kWalkCell;
+        const int team = cell ? e.teams[r].first : 1;
+        const int sets = e.teams[r].second;
+        // A one-warp run comes first.
+        const int beside = cell ? (r + 1 < runs ? kWalkLetsNext : 0) | (r > 0 ? kWalkWaitsLast : 0) : 0;
         if (team > 1) {
             TeamWalk a;
             a.nodes = w.nodes;
@@ -1670,20 +1684,22 @@ cudaError_t bh_ensemble_step(int64_t n, BHWorkspace &w, const BHEnsembleTables &
             a.work = work;
             a.params = e.params;
             a.P = w.P;
+            a.beside = beside;
             err = bh_team_walk(a, team, !e.all_soft, sets, st);
             if (err != cudaSuccess) return err;
         } else {
             const unsigned blocks = static_cast<unsigned>((static_cast<int64_t>(sets) * 32 + 255) / 256);
             if (w.counters)
                 launch_walk<true, false, true, true>(w, blocks, st, nullptr, Po, n, 0.f, 0.f, 0.f, P, Vo, Ao, nullptr,
-                                                     nullptr, w.counters, nullptr, 0, work, sets, e.params, w.P);
+                                                     nullptr, w.counters, nullptr, 0, work, sets, e.params, w.P, HostOut{}, beside);
             else if (e.all_soft)
                 launch_walk<false, false, true, false>(w, blocks, st, nullptr, Po, n, 0.f, 0.f, 0.f, P, Vo, Ao,
                                                        nullptr, nullptr, nullptr, nullptr, 0, work, sets, e.params,
-                                                       w.P);
+                                                       w.P, HostOut{}, beside);
             else
                 launch_walk<false, false, true, true>(w, blocks, st, nullptr, Po, n, 0.f, 0.f, 0.f, P, Vo, Ao, nullptr,
-                                                      nullptr, nullptr, nullptr, 0, work, sets, e.params, w.P);
+                                                      nullptr, nullptr, nullptr, 0, work, sets, e.params, w.P,
+                                                      HostOut{}, beside);
         }
         work += sets;
     }

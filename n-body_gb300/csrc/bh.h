@@ -140,9 +140,19 @@ struct TeamWalk {
     const float4 *params = nullptr;
     const uint32_t *P = nullptr;
     HostOut host;
+    int64_t first = 0;  // the system's first set
+    int beside = 0;     // kWalkLetsNext, kWalkWaitsLast
 };
+// Walks of one step side by side: launches that write different bodies and read
+// what no walk writes. Each but the last lets the next begin when its own last
+// CTAs have; each but the first begins without a wait and ends after the one
+// before (so that what follows the last follows all).
+constexpr int kWalkLetsNext = 1, kWalkWaitsLast = 2;
 // Warps per set of a system of n bodies: 1 is cell_walk_kernel.
 int bh_team_size(int64_t n);
+// The sets that bh_team_size walks; those after them are walked by teams of kTailTeam.
+int64_t bh_main_sets(int64_t n);
+constexpr int kTailTeam = 8;
 cudaError_t bh_team_walk(const TeamWalk &a, int team, bool guard, int64_t sets, cudaStream_t st);
 // Potential -sum m / sqrt(d^2 + eps^2) of every sorted body over the same
 // accepted records as the forces, into phi_out[ids[b]] (or phi_out[b]).

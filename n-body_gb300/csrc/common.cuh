@@ -102,6 +102,10 @@ __device__ __forceinline__ void tma_bulk_g2s(void *dst_smem, const void *src_gme
 // launched otherwise. Every access to memory they touch comes after it.
 __device__ __forceinline__ void wait_for_launches_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// Lets the kernel launched behind this one begin when every CTA of this one has
+// come here or ended, instead of when all have ended.
+__device__ __forceinline__ void let_next_launch_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // 1/sqrt(x), hardware approximation, flush-to-zero (inputs here are >= eps^2).
 __device__ __forceinline__ float rsqrt_ftz(float x) {
     float y;

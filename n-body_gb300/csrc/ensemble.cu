@@ -338,7 +338,7 @@ int relayout(nbody_ensemble *e) {
     if (!bh.empty()) {
         std::vector<int> seg(static_cast<size_t>(bh_n));
         std::vector<int4> chunks, warps;
-        std::vector<std::pair<int, int>> teams;
+        std::map<int, std::vector<int4>> by_team;  // the walk's sets by team size, each system's in order
         std::vector<int> fdepth(bh.size());
         std::vector<float4> prm(bh.size());
         for (size_t g = 0; g < bh.size(); ++g) {
@@ -349,12 +349,17 @@ int relayout(nbody_ensemble *e) {
             for (int c = 0; c < nch; ++c)
                 chunks.push_back(make_int4(static_cast<int>(g), f + c * kBBoxChunk,
                                            std::min(end, f + (c + 1) * kBBoxChunk), nch));
-            for (int b = f; b < end; b += kWarpBodies) warps.push_back(make_int4(static_cast<int>(g), b, f, end));
-            const int team = nbody::bh_team_size(s.n), sets = static_cast<int>((s.n + kWarpBodies - 1) / kWarpBodies);
-            if (teams.empty() || teams.back().first != team) teams.emplace_back(team, 0);
-            teams.back().second += sets;
+            const int tail = f + static_cast<int>(std::min(nbody::bh_main_sets(s.n) * kWarpBodies, s.n));
+            for (int b = f; b < end; b += kWarpBodies)
+                by_team[b < tail ? nbody::bh_team_size(s.n) : nbody::kTailTeam].push_back(
+                    make_int4(static_cast<int>(g), b, f, end));
             fdepth[g] = nbody::bh_father_depth(s.n);
             prm[g] = make_float4(s.dt, s.eps2, s.theta2, s.euler ? 1.f : 0.f);
+        }
+        std::vector<std::pair<int, int>> teams;
+        for (const auto &[team, sets] : by_team) {
+            teams.emplace_back(team, static_cast<int>(sets.size()));
+            warps.insert(warps.end(), sets.begin(), sets.end());
         }
         const size_t nsys = bh.size();
         const size_t bytes = bytes_of<int>(seg.size()) + bytes_of<int4>(chunks.size()) + bytes_of<unsigned>(8 * nsys) +

@@ -113,10 +113,11 @@ __global__ void __launch_bounds__(32 * W, W >= 16 && !SEG ? 1 : 32 / W) team_wal
     const float4 *__restrict__ pos, int64_t n, float eps2, float theta2, float dt, float4 *__restrict__ pos_out,
     float4 *__restrict__ vel, float4 *__restrict__ acc, float4 *__restrict__ force_out, const int *__restrict__ ids,
     unsigned long long *__restrict__ counters, int euler, const int4 *__restrict__ work,
-    const float4 *__restrict__ params, const uint32_t *__restrict__ P, const HostOut host) {
+    const float4 *__restrict__ params, const uint32_t *__restrict__ P, const HostOut host, int64_t first, int beside) {
     __shared__ __align__(16) TeamArea<W> A;
     constexpr int S = TeamArea<W>::S;
-    wait_for_launches_before();
+    if (!(beside & kWalkWaitsLast)) wait_for_launches_before();
+    if (beside & kWalkLetsNext) let_next_launch_begin();
     unsigned long long n_pairs = 0, n_visits = 0;
     float phi = 0.f;  // no potential in this form
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -132,7 +133,7 @@ __global__ void __launch_bounds__(32 * W, W >= 16 && !SEG ? 1 : 32 / W) team_wal
         root = static_cast<int>(P[ww.z]);
         rend = static_cast<int>(P[ww.w]);
     } else {
-        base = static_cast<int64_t>(blockIdx.x) * 64;
+        base = (first + blockIdx.x) * 64;
         end = n;
         root = 0;
         rend = static_cast<int>(*node_total);
@@ -329,6 +330,7 @@ __global__ void __launch_bounds__(32 * W, W >= 16 && !SEG ? 1 : 32 / W) team_wal
     A.sums[warp][2][lane] = fz.x;
     A.sums[warp][2][lane + 32] = fz.y;
     __syncthreads();
+    if ((beside & kWalkWaitsLast) && blockIdx.x == gridDim.x - 1) wait_for_launches_before();
     const int t = threadIdx.x;
     if (t >= 64) return;
     float gx = 0.f, gy = 0.f, gz = 0.f;
@@ -355,7 +357,7 @@ cudaError_t launch_form(const TeamWalk &a, unsigned sets, cudaStream_t st) {
     const auto launch = [&](auto kernel) {
         return launch_behind(kernel, dim3(sets), dim3(32 * W), 0, st, a.nodes, a.kids, a.node_total, a.pos, a.n, a.eps2,
                              a.theta2, a.dt, a.pos_out, a.vel, a.acc, a.force_out, a.ids, a.counters, a.euler, a.work,
-                             a.params, a.P, a.host);
+                             a.params, a.P, a.host, a.first, a.beside);
     };
     if constexpr (!SEG)
         if (a.host.pos) return launch(team_walk_kernel<W, COUNT, SEG, GUARD, true>);
@@ -386,12 +388,33 @@ cudaError_t launch_team(const TeamWalk &a, bool guard, unsigned sets, cudaStream
 // 10.6, 16 warps 12.4 ms per walk): 4 from 32,768 on although 8 is level with
 // it for one system up to 2^17, and 16 only below the sizes at which ensembles
 // turn to Barnes-Hut.
+constexpr int64_t kMaxTeams = 458752;  // with the tails below: 393,216 bodies 1.357 by fours, 1.381 ms by one warp
 int bh_team_size(int64_t n) {
     if (const char *e = std::getenv("NBODY_BH_TEAM")) {  // 1, 2, 4, 8 or 16: that team for every size
         const int v = std::atoi(e);
         if (v == 1 || v == 2 || v == 4 || v == 8 || v == 16) return v;
     }
-    return n < 10240 ? 16 : n < (1 << 15) ? 8 : n <= (1 << 19) ? 4 : 1;
+    return n < 10240 ? 16 : n < (1 << 15) ? 8 : n <= kMaxTeams ? 4 : 1;
+}
+
+// The last sets of a large system go to a launch of their own, by teams of 8,
+// that starts when the last CTAs of the others have: a set walked by one warp
+// takes 1.4 ms of a 3.2 ms walk of 2^20 bodies, so the SMs ran empty for a good
+// part of it. Walk of one Plummer system (GB300, ms), all sets alike / with the
+// tail: 131,073 bodies .527 / .498, 262,144 .961 / .922, 393,216 1.385 / 1.357,
+// 524,288 1.865 (4 warps: 1.808) / 1.686, 2^20 3.240 / 3.064, 2^21 6.115 / 5.970,
+// 2^22 12.19 / 12.01; a ball of 2^20 1.491 / 1.454. Behind teams of 4, 600 or 800
+// sets are level with 400; behind single warps 2,100 or 2,700 with 2,432 (16 per
+// SM). Tails by teams of 4 gain nothing, by teams of 16 half as much. Not up to
+// 2^17 bodies: the systems of an ensemble fill each other's ends, and teams of 8
+// cost 7 % more than teams of 4 there; which set is walked how follows from n
+// alone, so that a system sums in the same order in an ensemble.
+constexpr int64_t kTailMinBodies = 1 << 17;
+constexpr int64_t kTailSetsTeams = 400, kTailSetsOne = 2432;
+int64_t bh_main_sets(int64_t n) {
+    const int64_t sets = (n + 63) / 64;
+    if (n <= kTailMinBodies || std::getenv("NBODY_BH_TEAM")) return sets;
+    return (sets - (n <= kMaxTeams ? kTailSetsTeams : kTailSetsOne)) & ~int64_t(7);  // whole CTAs of cell_walk_kernel
 }
 
 cudaError_t bh_team_walk(const TeamWalk &a, int team, bool guard, int64_t sets, cudaStream_t st) {

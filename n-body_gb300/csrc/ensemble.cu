@@ -350,9 +350,10 @@ int relayout(nbody_ensemble *e) {
                 chunks.push_back(make_int4(static_cast<int>(g), f + c * kBBoxChunk,
                                            std::min(end, f + (c + 1) * kBBoxChunk), nch));
             const int tail = f + static_cast<int>(std::min(nbody::bh_main_sets(s.n) * kWarpBodies, s.n));
-            for (int b = f; b < end; b += kWarpBodies)
-                by_team[b < tail ? nbody::bh_team_size(s.n) : nbody::kTailTeam].push_back(
-                    make_int4(static_cast<int>(g), b, f, end));
+            std::vector<int4> &first = by_team[nbody::bh_team_size(s.n)];
+            for (int b = f; b < tail; b += kWarpBodies) first.push_back(make_int4(static_cast<int>(g), b, f, end));
+            std::vector<int4> *last = tail < end ? &by_team[nbody::kTailTeam] : nullptr;
+            for (int b = tail; b < end; b += kWarpBodies) last->push_back(make_int4(static_cast<int>(g), b, f, end));
             fdepth[g] = nbody::bh_father_depth(s.n);
             prm[g] = make_float4(s.dt, s.eps2, s.theta2, s.euler ? 1.f : 0.f);
         }

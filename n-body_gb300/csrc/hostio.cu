@@ -8,6 +8,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "launch.h"
 
 namespace nbody {
 
@@ -19,6 +20,7 @@ __global__ void host_gather_kernel(const float4 *__restrict__ positions4, const 
                                    const float4 *__restrict__ vel_h, const float4 *__restrict__ acc_h,
                                    float4 *__restrict__ pos_mass, float4 *__restrict__ vel,
                                    float4 *__restrict__ acc, int64_t n) {
+    wait_for_launches_before();
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 p = positions4[i];
@@ -30,6 +32,7 @@ __global__ void host_gather_kernel(const float4 *__restrict__ positions4, const 
 // inv[ids[i]] = i: the inverse of the sorted order's body ids (inv is filled
 // with -1 first, so an id that no body carries stays detectable).
 __global__ void invert_ids_kernel(const int *__restrict__ ids, int *__restrict__ inv, int64_t n, int *status) {
+    wait_for_launches_before();
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int d = ids[i];
@@ -57,6 +60,7 @@ __global__ void host_scatter_kernel(const float4 *__restrict__ pos_mass, const f
                                     float4 *__restrict__ positions4, float4 *__restrict__ vel_h,
                                     float4 *__restrict__ acc_h, float4 *__restrict__ force_h,
                                     float4 *__restrict__ masses_h, int64_t n, int *status) {
+    wait_for_launches_before();
     const int64_t d = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (d >= n) return;
     const int64_t i = inv ? inv[d] : d;
@@ -152,7 +156,7 @@ cudaError_t merge_masses(float4 *pos_mass, const float4 *masses4, int64_t n, cud
     if (n <= 0) return cudaSuccess;
     const int threads = 256;
     merge_masses_kernel<<<static_cast<unsigned>((n + threads - 1) / threads), threads, 0, stream>>>(pos_mass, masses4,
-                                                                                                   n);
+                                                                                                    n);
     return cudaGetLastError();
 }
 
@@ -160,8 +164,8 @@ cudaError_t host_gather(const float4 *positions4, const float4 *masses4, const f
                         float4 *pos_mass, float4 *vel, float4 *acc, int64_t n, cudaStream_t stream) {
     if (n <= 0) return cudaSuccess;
     const int threads = 256;
-    host_gather_kernel<<<static_cast<unsigned>((n + threads - 1) / threads), threads, 0, stream>>>(
-        positions4, masses4, vel_h, acc_h, pos_mass, vel, acc, n);
+    launch_behind(host_gather_kernel, dim3(static_cast<unsigned>((n + threads - 1) / threads)), dim3(threads), 0,
+                  stream, positions4, masses4, vel_h, acc_h, pos_mass, vel, acc, n);
     return cudaGetLastError();
 }
 
@@ -174,10 +178,10 @@ cudaError_t host_scatter(const float4 *pos_mass, const float4 *vel, const float4
     if (ids) {
         cudaError_t e = cudaMemsetAsync(inv, 0xff, static_cast<size_t>(n) * sizeof(int), stream);
         if (e != cudaSuccess) return e;
-        invert_ids_kernel<<<blocks, threads, 0, stream>>>(ids, inv, n, status);
+        launch_behind(invert_ids_kernel, dim3(blocks), dim3(threads), 0, stream, ids, inv, n, status);
     }
-    host_scatter_kernel<<<blocks, threads, 0, stream>>>(pos_mass, vel, acc, ids ? inv : nullptr, positions4, vel_h,
-                                                        acc_h, force_h, masses_h, n, status);
+    launch_behind(host_scatter_kernel, dim3(blocks), dim3(threads), 0, stream, pos_mass, vel, acc,
+                  ids ? inv : nullptr, positions4, vel_h, acc_h, force_h, masses_h, n, status);
     return cudaGetLastError();
 }
 

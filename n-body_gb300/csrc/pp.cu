@@ -29,6 +29,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "launch.h"
 #include "pp_common.cuh"
 
 namespace nbody {
@@ -48,6 +49,7 @@ template <int K, int T, bool GUARD>
 __global__ void __launch_bounds__(T, pp_min_blocks<K>())
     pp_force_kernel(const float4 *__restrict__ pos, int64_t n, float eps2, int nslices,
                     float4 *__restrict__ partial, unsigned *__restrict__ arrivals, Integrate g, int *status) {
+    wait_for_launches_before();
     // tile: TMA landing zone, bodies as float4 (x, y, z, m).
     // pairs: two tiles re-laid as j-pairs {x0 x1 y0 y1}{z0 z1 m0 m1}, so that
     // one 16-byte shared load yields two packed f32x2 operands.
@@ -244,6 +246,7 @@ template <int K, int T, bool GUARD>
 __global__ void __launch_bounds__(T, pp_min_blocks<K>())
     pp_force_linear_kernel(const float4 *__restrict__ pos, int64_t n, float eps2, float4 *__restrict__ partial,
                            unsigned *__restrict__ arrivals, Integrate g, int *status) {
+    wait_for_launches_before();
     __shared__ __align__(128) float4 tile[kPPStages][kPPTile];
     __shared__ __align__(128) float4 pairs[kPPTile];
     __shared__ __align__(8) uint64_t full[kPPStages];
@@ -576,18 +579,20 @@ static cudaError_t launch_kt(const PPPlan &plan, const float4 *pos, int64_t n, f
                              float4 *partial, unsigned *arrivals, cudaStream_t stream, int *status) {
     if (plan.linear_ctas > 0) {
         if (eps2 > 0.f)
-            pp_force_linear_kernel<K, T, false>
-                <<<plan.linear_ctas, T, 0, stream>>>(pos, n, eps2, partial, arrivals, g, status);
+            launch_behind(pp_force_linear_kernel<K, T, false>, dim3(plan.linear_ctas), dim3(T), 0, stream, pos, n,
+                          eps2, partial, arrivals, g, status);
         else
-            pp_force_linear_kernel<K, T, true>
-                <<<plan.linear_ctas, T, 0, stream>>>(pos, n, eps2, partial, arrivals, g, status);
+            launch_behind(pp_force_linear_kernel<K, T, true>, dim3(plan.linear_ctas), dim3(T), 0, stream, pos, n,
+                          eps2, partial, arrivals, g, status);
         return cudaGetLastError();
     }
     const dim3 grid(plan.iblocks, plan.slices);
     if (eps2 > 0.f)
-        pp_force_kernel<K, T, false><<<grid, T, 0, stream>>>(pos, n, eps2, plan.slices, partial, arrivals, g, status);
+        launch_behind(pp_force_kernel<K, T, false>, grid, dim3(T), 0, stream, pos, n, eps2, plan.slices, partial,
+                      arrivals, g, status);
     else
-        pp_force_kernel<K, T, true><<<grid, T, 0, stream>>>(pos, n, eps2, plan.slices, partial, arrivals, g, status);
+        launch_behind(pp_force_kernel<K, T, true>, grid, dim3(T), 0, stream, pos, n, eps2, plan.slices, partial,
+                      arrivals, g, status);
     return cudaGetLastError();
 }
 

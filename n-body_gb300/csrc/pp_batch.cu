@@ -15,6 +15,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "launch.h"
 #include "pp_batch.h"
 #include "pp_common.cuh"
 
@@ -64,6 +65,7 @@ __global__ void __launch_bounds__(T, K >= 4 ? 1 : 0)
                     float4 *__restrict__ acc, const int2 *__restrict__ items, int nitems,
                     const int4 *__restrict__ sys_range, const float4 *__restrict__ sys_prm,
                     unsigned *__restrict__ sched, int *status) {
+    wait_for_launches_before();
     __shared__ __align__(128) float4 tile[kPPStages][kPPTile];
     __shared__ __align__(128) float4 pairs[kPPTile];
     __shared__ __align__(8) uint64_t full[kPPStages];
@@ -145,20 +147,20 @@ cudaError_t pp_batch_launch(int shape, int ctas, const float4 *pos, float4 *pos_
     if (nitems <= 0 || ctas <= 0) return cudaSuccess;
     switch (shape) {
         case kPPBatch128x2:
-            pp_batch_kernel<2, 128><<<ctas, 128, 0, st>>>(pos, pos_out, vel, acc, items, nitems, sys_range, sys_prm,
-                                                          sched, status);
+            launch_behind(pp_batch_kernel<2, 128>, dim3(ctas), dim3(128), 0, st, pos, pos_out, vel, acc, items,
+                          nitems, sys_range, sys_prm, sched, status);
             break;
         case kPPBatch128x4:
-            pp_batch_kernel<4, 128><<<ctas, 128, 0, st>>>(pos, pos_out, vel, acc, items, nitems, sys_range, sys_prm,
-                                                          sched, status);
+            launch_behind(pp_batch_kernel<4, 128>, dim3(ctas), dim3(128), 0, st, pos, pos_out, vel, acc, items,
+                          nitems, sys_range, sys_prm, sched, status);
             break;
         case kPPBatch256x4:
-            pp_batch_kernel<4, 256><<<ctas, 256, 0, st>>>(pos, pos_out, vel, acc, items, nitems, sys_range, sys_prm,
-                                                          sched, status);
+            launch_behind(pp_batch_kernel<4, 256>, dim3(ctas), dim3(256), 0, st, pos, pos_out, vel, acc, items,
+                          nitems, sys_range, sys_prm, sched, status);
             break;
         default:
-            pp_batch_kernel<2, 256><<<ctas, 256, 0, st>>>(pos, pos_out, vel, acc, items, nitems, sys_range, sys_prm,
-                                                          sched, status);
+            launch_behind(pp_batch_kernel<2, 256>, dim3(ctas), dim3(256), 0, st, pos, pos_out, vel, acc, items,
+                          nitems, sys_range, sys_prm, sched, status);
             break;
     }
     return cudaGetLastError();

@@ -151,6 +151,7 @@ __global__ void __launch_bounds__(kSymT, kSymPerSm)
     const int range = blockIdx.x;
     const int x0 = p.begin[range], x1 = p.begin[range + 1];
     const float2 e2 = f2(eps2, eps2);
+    wait_for_launches_before();
     // Tile x: block b's own tiles, then those of blocks b + 1, b + 2, ... (cyclic).
     auto tile_first = [&](int x, int b) -> int64_t {
         const int t = x - sym_first(p, b);
@@ -439,9 +440,11 @@ cudaError_t pp_sym_launch(const SymPlan &p, const float4 *pos, int64_t n, float 
     float *rows = reinterpret_cast<float *>(static_cast<char *>(scratch) + p.parts_bytes);
     constexpr float lo = 8.2718061255302767e-25f /* 2^-80 */, hi = 9.6714065569170334e24f /* 2^83 */;
     if (eps2 >= lo && eps2 <= hi)
-        pp_sym_kernel<false><<<p.ctas, kSymT, 0, stream>>>(pos, n, eps2, p, parts, rows, status);
+        launch_behind(pp_sym_kernel<false>, dim3(p.ctas), dim3(kSymT), 0, stream, pos, n, eps2, p, parts, rows,
+                      status);
     else
-        pp_sym_kernel<true><<<p.ctas, kSymT, 0, stream>>>(pos, n, eps2, p, parts, rows, status);
+        launch_behind(pp_sym_kernel<true>, dim3(p.ctas), dim3(kSymT), 0, stream, pos, n, eps2, p, parts, rows,
+                      status);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     return launch_behind(pp_sym_sum_kernel, dim3(static_cast<unsigned>((n + kSymT - 1) / kSymT)), dim3(kSymT), 0, stream, pos,

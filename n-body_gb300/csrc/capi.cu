@@ -134,12 +134,23 @@ int fail(nbody_ctx *ctx, cudaError_t e) {
 
 bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-// Scratch for a direct-sum plan of n bodies, its arrival counters zero. Plans
-// of other sizes put partial sums where this one may have its counters, so
-// these are cleared when the plan's layout is not the one used last. A plan
-// that keeps every block's sums apart takes much more scratch than the others:
-// where that cannot be had the plan falls back.
+// Every plan's sums begin behind this much of the scratch, and its arrival
+// counters (zero before and after a launch) lie within: a launch of one plan, also
+// one replayed from a caller's graph, leaves the others' counters alone. Enough
+// for 8M bodies.
+constexpr size_t kArrivalsArea = 64 << 10;
+
+// Scratch for a direct-sum plan of n bodies, its arrival counters zero. Where a
+// plan's counters outgrow that area, they are cleared when the layout is not the
+// one used last. A plan that keeps every block's sums apart takes much more
+// scratch than the others: where that cannot be had the plan falls back.
 int ensure_scratch(nbody_ctx *ctx, int64_t n, nbody::PPPlan &plan) {
+    const auto reserve = [&] {
+        if (plan.partial_bytes == 0 || plan.arrivals_bytes >= kArrivalsArea) return;
+        plan.partial_bytes += kArrivalsArea - plan.arrivals_bytes;
+        plan.arrivals_bytes = kArrivalsArea;
+    };
+    reserve();
     for (;;) {
         if (plan.partial_bytes <= ctx->scratch_bytes) break;
         if (ctx->scratch) {
@@ -153,6 +164,7 @@ int ensure_scratch(nbody_ctx *ctx, int64_t n, nbody::PPPlan &plan) {
             cudaGetLastError();
             ctx->scratch = nullptr;
             plan = nbody::pp_plan(n, ctx->device, true, false);
+            reserve();
             continue;
         }
         NB_CK(ctx, e);
@@ -161,8 +173,7 @@ int ensure_scratch(nbody_ctx *ctx, int64_t n, nbody::PPPlan &plan) {
         ctx->scratch_arrivals = plan.arrivals_bytes;
     }
     if (plan.partial_bytes > 0 && plan.arrivals_bytes != ctx->scratch_arrivals) {
-        if (plan.arrivals_bytes > 0)
-            NB_CK(ctx, cudaMemsetAsync(ctx->scratch, 0, plan.arrivals_bytes, ctx->stream));
+        NB_CK(ctx, cudaMemsetAsync(ctx->scratch, 0, plan.arrivals_bytes, ctx->stream));
         ctx->scratch_arrivals = plan.arrivals_bytes;
     }
     return NBODY_OK;
@@ -384,6 +395,9 @@ bool pageable(std::initializer_list<const void *> arrays, size_t bytes) {
 // written, when it does).
 bool use_bounce(nbody_ctx *ctx, std::initializer_list<const void *> arrays) {
     if (ctx->n > kBounceBodies || ctx->bounce_failed) return false;
+    // A caller's graph reads and writes the arrays themselves when it is replayed.
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) return false;
     const size_t b4 = static_cast<size_t>(ctx->n) * sizeof(float4);
     if (!pageable(arrays, b4)) return false;
     if (!ctx->bounce) {

@@ -12,7 +12,7 @@ namespace nbody {
 // (14 launches): 184 -> 161 us; a host step of 4,096: 170 -> 167; ten resident
 // steps of 262,144: 11.41 -> 11.36 ms (GB300). Every kernel launched this way
 // waits in all its threads before it reads or writes memory, so a chain of them
-// is as ordered as plain launches.
+// is as ordered as plain launches (but for walks side by side: bh.h).
 template <class... Params, class... Args>
 cudaError_t launch_behind(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                           Args &&...args) {

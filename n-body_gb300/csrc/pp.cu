@@ -609,7 +609,8 @@ cudaError_t pp_launch(const PPPlan &plan, const float4 *pos, int64_t n, float ep
     if (plan.sym.blocks > 0) {
         if (!scratch) return cudaErrorInvalidValue;
         if (timer) timer->begin(kStagePPForce, stream);
-        const cudaError_t e = pp_sym_launch(plan.sym, pos, n, eps2, g, scratch, stream, status);
+        const cudaError_t e = pp_sym_launch(plan.sym, pos, n, eps2, g, static_cast<char *>(scratch) + plan.arrivals_bytes,
+                                            stream, status);
         if (timer) timer->end(kStagePPForce, stream);
         return e;
     }

@@ -461,10 +461,15 @@ def bench_bh(args, world, rank, local, dist):
     # bbox, keys, sort (a launch over tiles and one per merge pass up to 2^22
     # bodies, else histogram, scan, 8 passes), gather, 3 build kernels,
     # the upsweep (one climbing launch below 2^21 bodies; from there bucket
-    # centres, level count, level scatter and one launch per octree level: 24), walk
-    tiles = -(-n // (2048 if n <= 1 << 18 else 4096))
-    sort_launches = 10 if n > 1 << 22 else 1 + (tiles - 1).bit_length()
-    launches_per_step = 7 + sort_launches + (1 if n < (1 << 21) else 24)
+    # centres, level count, level scatter and one launch per octree level: 24),
+    # walk (from 2^17 bodies its last sets are a launch of their own)
+    sort_launches = 10
+    if n <= 1 << 22:
+        sort_launches, run = 1, 2048 if n <= 1 << 18 else 4096
+        while run < n:  # runs merged two at a time, up to 2^18 bodies four or (last) eight
+            run *= 2 if n > 1 << 18 else 8 if 4 * run < n <= 8 * run else 4
+            sort_launches += 1
+    launches_per_step = 6 + sort_launches + (1 if n < (1 << 21) else 24) + (1 if n <= 1 << 17 else 2)
     line = {"metric": METRIC, "component": "BH body-steps/s", "value": value, "unit": "body-steps/s",
             "n_gpus": world, "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms / args.steps,
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32", "data": "synthetic",

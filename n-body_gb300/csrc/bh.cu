@@ -1049,9 +1049,9 @@ constexpr int kCellDepth = 48;  // stack entries per warp; a full stack sends a 
 // 4.05 ms at 2^20 against 4.18 at twenty (48 registers) and 4.21 at
 // twenty-eight or thirty-two, 14.4 vs 15.4 ms at 4M (GB300, before the
 // children's cm moved to shared memory; with them there twenty still loses,
-// 4.0 vs 3.67 ms). An ensemble's
-// form also holds each system's eps^2 and theta^2 in registers and runs best
-// at sixteen (64 registers, no spills; 33.7 vs 30.8 ms at twenty for a
+// 4.0 vs 3.67 ms, and with redux boxes and a fused d^2, 3.43 vs 3.24). An
+// ensemble's form also holds each system's eps^2 and theta^2 in registers and
+// runs best at sixteen (64 registers, no spills; 33.7 vs 30.8 ms at twenty for a
 // 512-system ensemble). Against 256-thread CTAs at the same occupancy the
 // finer blocks shorten the uneven last wave (4.19 vs 4.28 ms at 2^20).
 template <bool COUNT, bool POT, bool SEG, bool GUARD, bool HOST = false>

@@ -385,9 +385,10 @@ cudaError_t launch_team(const TeamWalk &a, bool guard, unsigned sets, cudaStream
 // The size of a team follows from the system's size alone, so that it sums in
 // the same order in an ensemble, where fewer barriers count for more (128
 // ragged systems of up to 131,072 bodies: 1 warp 9.5, 4 warps 9.9, 8 warps
-// 10.6, 16 warps 12.4 ms per walk): 4 from 32,768 on although 8 is level with
-// it for one system up to 2^17, and 16 only below the sizes at which ensembles
-// turn to Barnes-Hut.
+// 10.6, 16 warps 12.4 ms per walk; 200 systems of 20,000: 1 warp 10.3, 8 warps
+// 11.7, 60 of 65,536: 1 warp 11.2, 4 warps 11.7): 4 from 32,768 on although 8 is
+// level with it for one system up to 2^17, and 16 only below the sizes at which
+// ensembles turn to Barnes-Hut.
 constexpr int64_t kMaxTeams = 458752;  // with the tails below: 393,216 bodies 1.357 by fours, 1.381 ms by one warp
 int bh_team_size(int64_t n) {
     if (const char *e = std::getenv("NBODY_BH_TEAM")) {  // 1, 2, 4, 8 or 16: that team for every size

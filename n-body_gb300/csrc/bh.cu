@@ -326,6 +326,7 @@ __global__ void keys_seg_kernel(const float4 *__restrict__ pos, int64_t n, const
 // Sort key of the segment passes: the system of the body now at slot j.
 __global__ void seg_keys_kernel(const uint32_t *__restrict__ vals, int64_t n, const int *__restrict__ seg,
                                 uint64_t *__restrict__ out, int *status) {
+    wait_for_launches_before();
     const int64_t j = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (j >= n) return;
     uint32_t v = vals[j];
@@ -343,7 +344,6 @@ __global__ void gather_kernel(const uint32_t *__restrict__ perm, int64_t n, cons
                               float4 *__restrict__ vel_out, float4 *__restrict__ acc_out,
                               int *__restrict__ id_out, int *status, const uint64_t *__restrict__ key_in,
                               uint64_t *__restrict__ key_out, uint32_t *__restrict__ mask) {
-    wait_for_launches_before();
     wait_for_launches_before();
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;

@@ -207,6 +207,7 @@ int nbody_set_key_mode(nbody_ctx *ctx, int mode);
  *
  * nbody_sort_pairs_device: sorts (uint64 key, uint32 value) pairs by key in
  * place, stably -- replaces src/shaders/ComputeShaders/bitonicSort.glsl:23-50.
+ * The arrays may begin at any key and value (8 and 4 bytes).
  *
  * nbody_bh_forces_device: Barnes-Hut accelerations of n bodies (library
  * layout, caller's order) with the context's eps2 and theta2: the

@@ -278,7 +278,10 @@ cudaError_t sort_pairs(uint64_t *keys, uint32_t *vals, uint64_t *keys_alt, uint3
     cudaError_t e = cudaGetDevice(&device);
     if (e == cudaSuccess) e = sort_prepare(device);
     if (e != cudaSuccess) return e;
-    if (passes == kPasses && sort_by_merging(n)) return merge_sort_pairs(keys, vals, keys_alt, vals_alt, n, stream);
+    // A caller's arrays may begin anywhere a key and a value may: the radix
+    // passes take them one by one (2^20 pairs: 212 us against 121 by merging).
+    if (passes == kPasses && sort_by_merging(n) && merge_sort_takes(keys, vals, keys_alt, vals_alt, n))
+        return merge_sort_pairs(keys, vals, keys_alt, vals_alt, n, stream);
     const int64_t tiles = (n + kTile - 1) / kTile;
     uint32_t *hist = static_cast<uint32_t *>(scratch);
     uint32_t *counters = hist + kPasses * kBins;

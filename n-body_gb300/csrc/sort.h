@@ -22,7 +22,10 @@ cudaError_t sort_prepare(int device);
 // The merge sort (sort_merge.cu) that sort_pairs takes for full keys of up to
 // some size: same result, always left in keys / vals, no scratch.
 bool sort_by_merging(int64_t n);
-// Kernel launches of sort_pairs.
+// Whether it takes arrays that begin at these addresses (sort_merge.cu).
+bool merge_sort_takes(const uint64_t *keys, const uint32_t *vals, const uint64_t *keys_alt, const uint32_t *vals_alt,
+                      int64_t n);
+// Kernel launches of sort_pairs (on arrays that the merge sort takes).
 int sort_launches(int64_t n, int passes = 8);
 int merge_sort_launches(int64_t n);
 cudaError_t merge_sort_prepare();

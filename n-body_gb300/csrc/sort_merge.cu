@@ -306,6 +306,16 @@ cudaError_t merge_sort_prepare() {
     return e == cudaSuccess ? prepare_block<512, 8>() : e;
 }
 
+// The passes of two runs store 16 bytes at a time, into either pair of arrays;
+// the others move single keys and values.
+bool merge_sort_takes(const uint64_t *keys, const uint32_t *vals, const uint64_t *keys_alt, const uint32_t *vals_alt,
+                      int64_t n) {
+    if (merge_ways(n, tile_of(n)) != 2) return true;
+    const uintptr_t all = reinterpret_cast<uintptr_t>(keys) | reinterpret_cast<uintptr_t>(vals) |
+                          reinterpret_cast<uintptr_t>(keys_alt) | reinterpret_cast<uintptr_t>(vals_alt);
+    return (all & 15u) == 0;
+}
+
 cudaError_t merge_sort_pairs(uint64_t *keys, uint32_t *vals, uint64_t *keys_alt, uint32_t *vals_alt, int64_t n,
                              cudaStream_t stream) {
     const int64_t tile = tile_of(n);

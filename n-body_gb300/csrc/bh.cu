@@ -46,28 +46,11 @@
 #include "common.cuh"
 #include "launch.h"
 #include "sort.h"
+#include "tree_links.cuh"
 
 namespace nbody {
 
 namespace {
-
-constexpr int kMaxLevel = 21;
-
-__device__ __forceinline__ int level_of(int delta) {
-    const int l = delta / 3;
-    return l < kMaxLevel ? l : kMaxLevel;
-}
-
-// Several systems packed back to back (an ensemble) are told apart by the
-// per-body system id sv.seg. The radix tree then runs over the composite keys
-// (system id as 32 leading bits, then the 63-bit key, then the index), so
-// delta between bodies of different systems is below 32 and inside a system it
-// is 32 + the key's delta. Nodes with delta < 32 join systems and are no
-// octree cell (level -1); below them each system's subtree is exactly the tree
-// of that system alone. sv.seg == nullptr is the single-system solver.
-__device__ __forceinline__ int level_c(int delta, int base) {
-    return delta < base ? -1 : level_of(delta - base);
-}
 
 __device__ __forceinline__ bool same_key(const uint64_t *__restrict__ k, const SegView &sv, int64_t a, int64_t b) {
     return k[a] == k[b] && (sv.seg == nullptr || sv.seg[a] == sv.seg[b]);
@@ -343,11 +326,13 @@ __global__ void gather_kernel(const uint32_t *__restrict__ perm, int64_t n, cons
                               const int *__restrict__ id_in, float4 *__restrict__ pos_out,
                               float4 *__restrict__ vel_out, float4 *__restrict__ acc_out,
                               int *__restrict__ id_out, int *status, const uint64_t *__restrict__ key_in,
-                              uint64_t *__restrict__ key_out, uint32_t *__restrict__ mask) {
+                              uint64_t *__restrict__ key_out, uint32_t *__restrict__ mask,
+                              unsigned *__restrict__ broken) {
     wait_for_launches_before();
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
     mask[i] = 0u;  // for the build that follows
+    if (i == 0) *broken = 0u;
     uint32_t j = perm[i];
     if (j >= static_cast<uint64_t>(n)) {  // not a permutation: report, read in bounds
         record_error(status, NBODY_ERR_CAPACITY);
@@ -377,10 +362,12 @@ __device__ __forceinline__ int delta_at(const uint64_t *__restrict__ k, const in
 
 // Also presets, for the kernels that follow, the scan's tile words, the child
 // table (two rows per thread: 2 n rows hold every record) and, with arrive set,
-// the climb's counters. n >= 1 threads.
+// the climb's counters. n >= 1 threads. Keys out of order (a sort that gave up)
+// raise *broken.
 __global__ void radix_tree_kernel(const uint64_t *__restrict__ k, int64_t n, BinaryTree t, SegView sv,
                                   uint32_t *__restrict__ mask, int base, unsigned long long *__restrict__ scan_words,
-                                  int scan_count, int4 *__restrict__ kids, unsigned *__restrict__ arrive) {
+                                  int scan_count, int4 *__restrict__ kids, unsigned *__restrict__ arrive,
+                                  unsigned *__restrict__ broken, int *status) {
     wait_for_launches_before();
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -391,6 +378,10 @@ __global__ void radix_tree_kernel(const uint64_t *__restrict__ k, int64_t n, Bin
     if (arrive) reinterpret_cast<uint2 *>(arrive)[i] = make_uint2(0u, 0u);
     if (i >= n - 1) return;
     const int *seg = sv.seg;
+    if (out_of_order(k, seg, i)) {
+        *broken = 1u;
+        record_error(status, NBODY_ERR_CAPACITY);
+    }
     const int dl = delta_at(k, seg, n, i, i - 1), dr = delta_at(k, seg, n, i, i + 1);
     const int d = dr > dl ? 1 : -1;
     const int dmin = d > 0 ? dl : dr;
@@ -444,7 +435,7 @@ constexpr unsigned long long kScanCount = 1ull << 62, kScanPrefix = 2ull << 62, 
 __global__ void __launch_bounds__(kScanThreads) count_scan_kernel(const uint64_t *__restrict__ k, int64_t n,
                                                                   const uint32_t *__restrict__ mask, SegView sv,
                                                                   uint32_t *__restrict__ P, unsigned long long *words,
-                                                                  int *status) {
+                                                                  unsigned *__restrict__ broken, int *status) {
     wait_for_launches_before();
     __shared__ uint32_t warp_sums[kScanThreads / 32];
     __shared__ unsigned s_tile;
@@ -497,6 +488,7 @@ __global__ void __launch_bounds__(kScanThreads) count_scan_kernel(const uint64_t
                 for (uint32_t spin = 0; !((w = vw[mine]) & ~kScanValue);)
                     if (++spin >= kWaitSpinCap || ((spin & 1023u) == 0 && global_ns() - t0 > kWaitLimitNs)) {
                         record_error(status, NBODY_ERR_TIMEOUT);
+                        *broken = 1u;
                         w = kScanPrefix;
                         break;
                     }
@@ -545,53 +537,27 @@ __device__ __forceinline__ float cell_side2(uint64_t key, int L, const float *__
     return __fmul_rn(s, s);
 }
 
-// Record index of the cell whose top radix-tree node is p.
-__device__ __forceinline__ int record_of(const BinaryTree &t, const uint32_t *__restrict__ mask,
-                                         const uint32_t *__restrict__ P, int p, int base) {
-    const int L = level_c(t.delta[p], base);
-    const int lo = t.lo[p];
-    return static_cast<int>(P[lo] + __popc(mask[lo] & ((1u << L) - 1u)));
-}
-
-// Octree parent of a record: the nearest radix-tree ancestor that is a cell
-// top (the nodes in between split the same cell; at most 6 of them), or -1.
-__device__ __forceinline__ int parent_top(const BinaryTree &t, int p) {
-    // At most 6 nodes per octree level inside a system, and at most 32 joining
-    // nodes (strictly decreasing delta < 32) above a system's subtree.
-    for (int guard = 0; p >= 0 && !t.top[p] && guard < 160; ++guard) p = t.iparent[p];
-    return p >= 0 && t.top[p] ? p : -1;
-}
-
-// Record idx, whose bodies' first key is `key`, into its parent's row of the
-// child table (8 places per cell, by key digit, -1 before). p: its radix-tree
-// parent. Returns the parent record (-1: a root).
-__device__ __forceinline__ int link_child(const BinaryTree &t, const uint32_t *__restrict__ mask,
-                                          const uint32_t *__restrict__ P, int p, int base, uint64_t key, int idx,
-                                          int *__restrict__ kids) {
-    p = parent_top(t, p);
-    if (p < 0) return -1;
-    const int par = record_of(t, mask, P, p, base);
-    const int digit = static_cast<int>(key >> (63 - 3 * (level_c(t.delta[p], base) + 1))) & 7;
-    kids[8 * static_cast<int64_t>(par) + digit] = idx;
-    return par;
-}
-
 // The records: thread i writes the cell whose top is radix-tree node i, and
-// body i's leaf if it is a lone body.
+// body i's leaf if it is a lone body. Of a broken tree (keys out of order, or
+// prefix sums that were not waited for) every record is a leaf without a parent,
+// so that the upsweep and the walks that follow end at once.
 __global__ void emit_kernel(const uint64_t *__restrict__ k, int64_t n, const float4 *__restrict__ pos, BinaryTree t,
                             const uint32_t *__restrict__ mask, const uint32_t *__restrict__ P,
                             const float *__restrict__ box, BHNode *__restrict__ nodes, Records r, int *__restrict__ kids,
-                            SegView sv, bool parents) {
+                            SegView sv, bool parents, const unsigned *__restrict__ broken, int *status) {
     wait_for_launches_before();
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int base = sv.seg ? 32 : 0;
+    const bool whole = *broken == 0u;
     if (i < n - 1 && t.top[i]) {
         const int L = level_c(t.delta[i], base);
         const int lo = t.lo[i], hi = t.hi[i];
         const int idx = record_of(t, mask, P, static_cast<int>(i), base);
         int4 meta;
-        if (L < kMaxLevel) {
+        if (!whole) {
+            meta = make_int4(__float_as_int(-1.f), static_cast<int>(P[hi + 1]), lo, 1);
+        } else if (L < kMaxLevel) {
             meta = make_int4(__float_as_int(cell_side2(k[lo], L, box_of(sv, box, lo))), static_cast<int>(P[hi + 1]), lo,
                              0);
         } else {  // bucket of bodies with identical keys: a leaf
@@ -599,7 +565,8 @@ __global__ void emit_kernel(const uint64_t *__restrict__ k, int64_t n, const flo
         }
         nodes[idx].meta = meta;
         r.level[idx] = L;
-        const int par = i == 0 ? -1 : link_child(t, mask, P, t.iparent[i], base, k[lo], idx, kids);
+        const int par = i == 0 || !whole ? kNoParent : link_child(t, mask, P, t.iparent[i], base, k[lo], idx, kids);
+        if (par == kMisplaced) record_error(status, NBODY_ERR_CAPACITY);
         if (parents) r.parent[idx] = par;  // for the climbing upsweep
     }
     const bool lone = !((i > 0 && same_key(k, sv, i, i - 1)) || (i + 1 < n && same_key(k, sv, i, i + 1)));
@@ -608,7 +575,8 @@ __global__ void emit_kernel(const uint64_t *__restrict__ k, int64_t n, const flo
     nodes[idx].cm = pos[i];
     nodes[idx].meta = make_int4(__float_as_int(-1.f), static_cast<int>(P[i + 1]), static_cast<int>(i), 1);
     r.level[idx] = kMaxLevel + 1;  // a lone body
-    const int par = n < 2 ? -1 : link_child(t, mask, P, t.lparent[i], base, k[i], idx, kids);
+    const int par = n < 2 || !whole ? kNoParent : link_child(t, mask, P, t.lparent[i], base, k[i], idx, kids);
+    if (par == kMisplaced) record_error(status, NBODY_ERR_CAPACITY);
     if (parents) r.parent[idx] = par;
 }
 
@@ -1377,6 +1345,7 @@ size_t bh_workspace_layout(int64_t n, void *base, BHWorkspace *w) {
     w->box = static_cast<float *>(take(sizeof(float) * 8));
     w->bbox_partial = static_cast<float *>(take(sizeof(float) * 6 * kBBoxBlocks));
     w->bbox_counter = static_cast<unsigned *>(take(sizeof(unsigned) * 4));
+    w->broken = static_cast<unsigned *>(take(sizeof(unsigned)));
     w->tree.lo = static_cast<int *>(take(sizeof(int) * nn));
     w->tree.hi = static_cast<int *>(take(sizeof(int) * nn));
     w->tree.delta = static_cast<int *>(take(sizeof(int) * nn));
@@ -1439,7 +1408,7 @@ cudaError_t bh_gather(int64_t n, const BHWorkspace &w, const float4 *pos_in, con
                       int *id_out, cudaStream_t st, int *status, StageTimer *timer) {
     if (timer) timer->begin(kStageGather, st);
     launch_behind(gather_kernel, dim3(grid_for(n, 256)), dim3(256), 0, st, w.vals[0], n, pos_in, vel_in, acc_in,
-                  id_in, pos_out, vel_out, acc_out, id_out, status, nullptr, nullptr, w.mask);
+                  id_in, pos_out, vel_out, acc_out, id_out, status, nullptr, nullptr, w.mask, w.broken);
     if (timer) timer->end(kStageGather, st);
     return cudaGetLastError();
 }
@@ -1468,11 +1437,11 @@ cudaError_t bh_build(const float4 *pos_sorted, int64_t n, BHWorkspace &w, cudaSt
     const int tiles = static_cast<int>((n + kScanTile - 1) / kScanTile);
     launch_behind(radix_tree_kernel, dim3(grid_for(n, 256)), dim3(256), 0, st, k, n, w.tree, sv, w.mask,
                   sv.seg ? 32 : 0, w.scan_words, tiles + 1, reinterpret_cast<int4 *>(w.kids),
-                  levels ? nullptr : w.rec.arrive);
+                  levels ? nullptr : w.rec.arrive, w.broken, status);
     launch_behind(count_scan_kernel, dim3(tiles), dim3(kScanThreads), 0, st, k, n, w.mask, sv, w.P, w.scan_words,
-                  status);
+                  w.broken, status);
     launch_behind(emit_kernel, dim3(grid_for(n, 256)), dim3(256), 0, st, k, n, pos_sorted, w.tree, w.mask, w.P,
-                  w.box, w.nodes, w.rec, w.kids, sv, !levels);
+                  w.box, w.nodes, w.rec, w.kids, sv, !levels, w.broken, status);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     if (timer) timer->end(kStageBuild, st);
@@ -1651,7 +1620,7 @@ cudaError_t bh_ensemble_step(int64_t n, BHWorkspace &w, const BHEnsembleTables &
     // Sorted keys into keys[0] (the build reads them there), permutation in vals[0].
     uint64_t *ksorted = w.keys[0];
     launch_behind(gather_kernel, dim3(grid_for(n, 256)), dim3(256), 0, st, v0, n, P, V, A, I, Po, Vo, Ao, Io, status,
-                  e.keys_orig, ksorted, w.mask);
+                  e.keys_orig, ksorted, w.mask, w.broken);
     if (tm) tm->end(kStageGather, st);
     err = cudaGetLastError();
     if (err != cudaSuccess) return err;

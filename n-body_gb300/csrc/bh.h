@@ -70,6 +70,7 @@ struct BHWorkspace {
     uint32_t *mask = nullptr;
     uint32_t *P = nullptr;  // n + 1 entries; P[n] = record count
     unsigned long long *scan_words = nullptr;
+    unsigned *broken = nullptr;  // raised by a build whose keys or prefix sums are not whole; cleared by the gather
     BHNode *nodes = nullptr;  // up to 2n records
     int *kids = nullptr;      // child table: 8 places per cell record, by key digit; -1: no child
     // Traversal counters (pairwise evaluations, warp record visits): the

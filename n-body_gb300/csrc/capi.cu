@@ -21,6 +21,7 @@
 #include "init.h"
 #include "kernels.h"
 #include "nbody_gb300.h"
+#include "scratch.h"
 #include "sort.h"
 #include "timer.h"
 
@@ -70,9 +71,7 @@ struct nbody_ctx {
     float4 *bounce = nullptr;
     bool bounce_failed = false;
     bool bounce_read = false;  // work on the stream may still read it
-    void *scratch = nullptr;
-    size_t scratch_bytes = 0;
-    size_t scratch_arrivals = 0;  // bytes of arrival counters of the plan that used it last
+    nbody::PPScratch scratch;
     bool uploaded = false;
     nbody::EventTimer *timer = nullptr;  // non-null while profiling is enabled
     std::string last_error;
@@ -134,48 +133,25 @@ int fail(nbody_ctx *ctx, cudaError_t e) {
 
 bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-// Every plan's sums begin behind this much of the scratch, and its arrival
-// counters (zero before and after a launch) lie within: a launch of one plan, also
-// one replayed from a caller's graph, leaves the others' counters alone. Enough
-// for 8M bodies.
-constexpr size_t kArrivalsArea = 64 << 10;
+// The direct sum's plan for n bodies, and scratch for it.
+nbody::PPPlan plan_of(const nbody_ctx *ctx, int64_t n) {
+    return nbody::pp_scratch_plan(ctx->scratch, [&](bool sym) { return nbody::pp_plan(n, ctx->device, true, sym); });
+}
 
-// Scratch for a direct-sum plan of n bodies, its arrival counters zero. Where a
-// plan's counters outgrow that area, they are cleared when the layout is not the
-// one used last. A plan that keeps every block's sums apart takes much more
-// scratch than the others: where that cannot be had the plan falls back.
 int ensure_scratch(nbody_ctx *ctx, int64_t n, nbody::PPPlan &plan) {
-    const auto reserve = [&] {
-        if (plan.partial_bytes == 0 || plan.arrivals_bytes >= kArrivalsArea) return;
-        plan.partial_bytes += kArrivalsArea - plan.arrivals_bytes;
-        plan.arrivals_bytes = kArrivalsArea;
-    };
-    reserve();
-    for (;;) {
-        if (plan.partial_bytes <= ctx->scratch_bytes) break;
-        if (ctx->scratch) {
-            NB_CK(ctx, cudaStreamSynchronize(ctx->stream));
-            cudaFree(ctx->scratch);
-            ctx->scratch = nullptr;
-            ctx->scratch_bytes = 0;
+    struct {
+        cudaStream_t stream;
+        cudaError_t alloc(void **p, size_t bytes) {
+            const cudaError_t e = cudaMalloc(p, bytes);
+            if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+            return e;
         }
-        const cudaError_t e = cudaMalloc(&ctx->scratch, plan.partial_bytes);
-        if (e == cudaErrorMemoryAllocation && plan.sym.blocks > 0) {
-            cudaGetLastError();
-            ctx->scratch = nullptr;
-            plan = nbody::pp_plan(n, ctx->device, true, false);
-            reserve();
-            continue;
-        }
-        NB_CK(ctx, e);
-        NB_CK(ctx, cudaMemsetAsync(ctx->scratch, 0, plan.partial_bytes, ctx->stream));
-        ctx->scratch_bytes = plan.partial_bytes;
-        ctx->scratch_arrivals = plan.arrivals_bytes;
-    }
-    if (plan.partial_bytes > 0 && plan.arrivals_bytes != ctx->scratch_arrivals) {
-        NB_CK(ctx, cudaMemsetAsync(ctx->scratch, 0, plan.arrivals_bytes, ctx->stream));
-        ctx->scratch_arrivals = plan.arrivals_bytes;
-    }
+        cudaError_t clear(void *p, size_t bytes) { return cudaMemsetAsync(p, 0, bytes, stream); }
+        cudaError_t wait() { return cudaStreamSynchronize(stream); }
+        void free(void *p) { cudaFree(p); }
+    } device{ctx->stream};
+    NB_CK(ctx, nbody::pp_scratch_ensure(ctx->scratch, plan, device,
+                                        [&](bool sym) { return nbody::pp_plan(n, ctx->device, true, sym); }));
     return NBODY_OK;
 }
 
@@ -191,16 +167,16 @@ int read_status(nbody_ctx *ctx) {
         NB_CK(ctx, cudaStreamSynchronize(ctx->stream));
     }
     ctx->bounce_read = false;
-    if (h != NBODY_OK && ctx->scratch) {
+    if (h != NBODY_OK && ctx->scratch.mem) {
         // A kernel gave up part-way: its arrival counters may be left non-zero.
-        NB_CK(ctx, cudaMemsetAsync(ctx->scratch, 0, ctx->scratch_bytes, ctx->stream));
+        NB_CK(ctx, cudaMemsetAsync(ctx->scratch.mem, 0, ctx->scratch.bytes, ctx->stream));
         NB_CK(ctx, cudaStreamSynchronize(ctx->stream));
     }
     return h;
 }
 
 int pp_steps(nbody_ctx *ctx, int steps) {
-    nbody::PPPlan plan = nbody::pp_plan(ctx->n, ctx->device);
+    nbody::PPPlan plan = plan_of(ctx, ctx->n);
     int rc = ensure_scratch(ctx, ctx->n, plan);
     if (rc != NBODY_OK) return rc;
     for (int s = 0; s < steps; ++s) {
@@ -210,7 +186,7 @@ int pp_steps(nbody_ctx *ctx, int steps) {
         g.acc = ctx->acc;
         g.dt = ctx->dt;
         g.euler = ctx->integrator == NBODY_INTEGRATOR_GPU_EULER;
-        NB_CK(ctx, nbody::pp_launch(plan, ctx->pos[ctx->cur], ctx->n, ctx->eps2, g, ctx->scratch, ctx->stream,
+        NB_CK(ctx, nbody::pp_launch(plan, ctx->pos[ctx->cur], ctx->n, ctx->eps2, g, ctx->scratch.mem, ctx->stream,
                                     ctx->status, ctx->timer));
         ctx->cur ^= 1;
     }
@@ -543,7 +519,7 @@ int nbody_destroy(nbody_ctx *ctx) {
         if (ctx->status_host) cudaFreeHost(ctx->status_host);
         else cudaFree(ctx->status);
         if (ctx->bounce) cudaFreeHost(ctx->bounce);
-        cudaFree(ctx->scratch);
+        cudaFree(ctx->scratch.mem);
         cudaFree(ctx->vel2[1]);
         cudaFree(ctx->acc2[1]);
         cudaFree(ctx->ids[0]);
@@ -800,7 +776,7 @@ bool pp_update_graphed(nbody_ctx *ctx, const float *positions4, float *velocitie
            *ma = nbody::host_mapped(accelerations4, b4, dev), *mm = nbody::host_mapped(masses4, b4, dev);
     float4 *mf = forces4 ? nbody::host_mapped(forces4, b4, dev) : nullptr;
     if (!(mp && mv && ma && mm && (!forces4 || mf))) return false;
-    nbody::PPPlan plan = nbody::pp_plan(ctx->n, ctx->device);
+    nbody::PPPlan plan = plan_of(ctx, ctx->n);
     *rc = ensure_scratch(ctx, ctx->n, plan);  // allocation stays outside the capture
     if (*rc != NBODY_OK) return true;
     auto body = [&]() -> int {
@@ -811,14 +787,14 @@ bool pp_update_graphed(nbody_ctx *ctx, const float *positions4, float *velocitie
         g.acc = ctx->acc;
         g.dt = ctx->dt;
         g.euler = ctx->integrator == NBODY_INTEGRATOR_GPU_EULER;
-        NB_CK(ctx, nbody::pp_launch(plan, ctx->pos[0], ctx->n, ctx->eps2, g, ctx->scratch, ctx->stream, ctx->status,
+        NB_CK(ctx, nbody::pp_launch(plan, ctx->pos[0], ctx->n, ctx->eps2, g, ctx->scratch.mem, ctx->stream, ctx->status,
                                     nullptr));
         NB_CK(ctx, nbody::host_scatter(ctx->pos[1], ctx->vel, ctx->acc, nullptr, nullptr, mp, mv, ma, mf, nullptr,
                                        ctx->n, ctx->stream, ctx->status));
         return NBODY_OK;
     };
     GraphKey key = graph_key(ctx);
-    key.ws = ctx->scratch;
+    key.ws = ctx->scratch.mem;
     const void *arrays[9] = {mp, mv, ma, mm, mf, nullptr, nullptr, nullptr, nullptr};
     for (int i = 0; i < 9; ++i) key.host[i] = arrays[i];
     bool replayed = false;
@@ -982,12 +958,12 @@ int nbody_pp_forces_device(nbody_ctx *ctx, const void *pos_mass4, void *force4, 
     if (!ctx || !pos_mass4 || !force4 || n <= 0) return NBODY_ERR_ARG;
     if (!aligned16(pos_mass4) || !aligned16(force4)) return NBODY_ERR_ARG;
     DeviceGuard dg(ctx->device);
-    nbody::PPPlan plan = nbody::pp_plan(n, ctx->device);
+    nbody::PPPlan plan = plan_of(ctx, n);
     int rc = ensure_scratch(ctx, n, plan);
     if (rc != NBODY_OK) return rc;
     nbody::Integrate g;
     g.force = static_cast<float4 *>(force4);
-    NB_CK(ctx, nbody::pp_launch(plan, static_cast<const float4 *>(pos_mass4), n, ctx->eps2, g, ctx->scratch,
+    NB_CK(ctx, nbody::pp_launch(plan, static_cast<const float4 *>(pos_mass4), n, ctx->eps2, g, ctx->scratch.mem,
                                 ctx->stream, ctx->status, ctx->timer));
     return NBODY_OK;
 }
@@ -999,7 +975,7 @@ int nbody_pp_step_device(nbody_ctx *ctx, const void *pos_in, void *pos_out, void
         (force4 && !aligned16(force4)))
         return NBODY_ERR_ARG;
     DeviceGuard dg(ctx->device);
-    nbody::PPPlan plan = nbody::pp_plan(n, ctx->device);
+    nbody::PPPlan plan = plan_of(ctx, n);
     int rc = ensure_scratch(ctx, n, plan);
     if (rc != NBODY_OK) return rc;
     nbody::Integrate g;
@@ -1009,7 +985,7 @@ int nbody_pp_step_device(nbody_ctx *ctx, const void *pos_in, void *pos_out, void
     g.force = static_cast<float4 *>(force4);
     g.dt = ctx->dt;
     g.euler = ctx->integrator == NBODY_INTEGRATOR_GPU_EULER;
-    NB_CK(ctx, nbody::pp_launch(plan, static_cast<const float4 *>(pos_in), n, ctx->eps2, g, ctx->scratch,
+    NB_CK(ctx, nbody::pp_launch(plan, static_cast<const float4 *>(pos_in), n, ctx->eps2, g, ctx->scratch.mem,
                                 ctx->stream, ctx->status, ctx->timer));
     return NBODY_OK;
 }
@@ -1017,7 +993,7 @@ int nbody_pp_step_device(nbody_ctx *ctx, const void *pos_in, void *pos_out, void
 int nbody_pp_config(nbody_ctx *ctx, int64_t n, int *bodies_per_thread, int *slices, int *ctas) {
     if (!ctx || n <= 0) return NBODY_ERR_ARG;
     DeviceGuard dg(ctx->device);
-    const nbody::PPPlan plan = nbody::pp_plan(n, ctx->device);
+    const nbody::PPPlan plan = plan_of(ctx, n);
     if (bodies_per_thread) *bodies_per_thread = plan.k;
     if (slices) *slices = plan.slices;
     if (ctas) *ctas = plan.sym.blocks > 0 ? plan.sym.ctas : plan.linear_ctas > 0 ? plan.linear_ctas : plan.iblocks * plan.slices;

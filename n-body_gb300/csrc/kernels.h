@@ -79,6 +79,8 @@ PPPlan pp_plan_within(int64_t n, int device, size_t scratch_bytes);
 cudaError_t pp_launch(const PPPlan &plan, const float4 *pos, int64_t n, float eps2, const Integrate &g,
                       void *scratch, cudaStream_t stream, int *status, StageTimer *timer = nullptr);
 
+// The word in front of scratch is zero before; it is raised where a CTA's sums are not whole, and then
+// nothing is written.
 cudaError_t pp_sym_launch(const SymPlan &p, const float4 *pos, int64_t n, float eps2, const Integrate &g, void *scratch,
                           cudaStream_t stream, int *status);
 

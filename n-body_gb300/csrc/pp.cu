@@ -470,7 +470,8 @@ PPPlan pp_plan(int64_t n, int device, bool allow_linear, bool allow_sym) {
             p.threads = 256;
             p.iblocks = p.sym.blocks;
             p.slices = p.sym.ctas / p.sym.blocks;
-            p.partial_bytes = p.sym.bytes;
+            p.arrivals_bytes = 256;  // its last word: a CTA gave up
+            p.partial_bytes = p.arrivals_bytes + p.sym.bytes;
             return p;
         }
     }

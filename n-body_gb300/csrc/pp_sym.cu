@@ -306,10 +306,12 @@ __global__ void __launch_bounds__(kSymT, kSymPerSm)
     }
     if (failed) {
         // Drain this CTA's copies still in flight before shared memory goes away.
-        if (tid == 0)
+        if (tid == 0) {
+            parts[-1] = 1.f;
             for (int u = fail_at; u < x1 && u < fail_at + kSymStages; ++u)
                 mbar_wait_bounded(&S.full[(u - x0) % kSymStages], static_cast<uint32_t>((u - x0) / kSymStages) & 1u,
                                   status);
+        }
         __syncthreads();
         return;
     }
@@ -319,7 +321,9 @@ __global__ void __launch_bounds__(kSymT, kSymPerSm)
 // The sum of each body, one thread per body: the parts of the ranges that held
 // its block, in order, then the j-rows that met it, in order of distance; then
 // the integrator. A kernel of its own, over the whole chip: the last CTA of
-// each block doing it in pp_sym_kernel took 15 us at 16,384 bodies.
+// each block doing it in pp_sym_kernel took 15 us at 16,384 bodies. Where a CTA
+// gave up (parts[-1]), its parts and rows are those of an earlier call, and
+// nothing is written until the status has been reported and the word cleared.
 __global__ void __launch_bounds__(kSymT) pp_sym_sum_kernel(const float4 *__restrict__ pos, int64_t n,
                                                            const __grid_constant__ SymPlan p,
                                                            const float *__restrict__ parts,
@@ -379,6 +383,7 @@ __global__ void __launch_bounds__(kSymT) pp_sym_sum_kernel(const float4 *__restr
             fz += vz[u];
         }
     }
+    if (parts[-1] != 0.f) return;
     if (g.pos_out) integrate_body(i, pos[i], fx, fy, fz, g);
     else if (g.force) g.force[i] = make_float4(fx, fy, fz, 0.f);
 }

@@ -70,7 +70,8 @@ struct nbody_ctx {
     // arrays of n float4; made on first use).
     float4 *bounce = nullptr;
     bool bounce_failed = false;
-    bool bounce_read = false;  // work on the stream may still read it
+    bool bounce_read = false;        // work in front of bounce_free may still use it
+    cudaEvent_t bounce_free = nullptr;  // on the stream that the work went to (nbody_set_stream may change it)
     nbody::PPScratch scratch;
     bool uploaded = false;
     nbody::EventTimer *timer = nullptr;  // non-null while profiling is enabled
@@ -166,7 +167,6 @@ int read_status(nbody_ctx *ctx) {
         NB_CK(ctx, cudaMemsetAsync(ctx->status, 0, sizeof(int), ctx->stream));
         NB_CK(ctx, cudaStreamSynchronize(ctx->stream));
     }
-    ctx->bounce_read = false;
     if (h != NBODY_OK && ctx->scratch.mem) {
         // A kernel gave up part-way: its arrival counters may be left non-zero.
         NB_CK(ctx, cudaMemsetAsync(ctx->scratch.mem, 0, ctx->scratch.bytes, ctx->stream));
@@ -377,16 +377,26 @@ bool use_bounce(nbody_ctx *ctx, std::initializer_list<const void *> arrays) {
     const size_t b4 = static_cast<size_t>(ctx->n) * sizeof(float4);
     if (!pageable(arrays, b4)) return false;
     if (!ctx->bounce) {
-        if (cudaHostAlloc(reinterpret_cast<void **>(&ctx->bounce), 5 * b4, cudaHostAllocMapped) != cudaSuccess) {
+        if (!ctx->bounce_free && cudaEventCreateWithFlags(&ctx->bounce_free, cudaEventDisableTiming) != cudaSuccess)
+            ctx->bounce_free = nullptr;
+        if (!ctx->bounce_free ||
+            cudaHostAlloc(reinterpret_cast<void **>(&ctx->bounce), 5 * b4, cudaHostAllocMapped) != cudaSuccess) {
             cudaGetLastError();
             ctx->bounce = nullptr;
             ctx->bounce_failed = true;
             return false;
         }
     }
-    if (ctx->bounce_read && cudaStreamSynchronize(ctx->stream) != cudaSuccess) return false;
+    if (ctx->bounce_read && cudaEventSynchronize(ctx->bounce_free) != cudaSuccess) return false;
     ctx->bounce_read = false;
     return true;
+}
+
+// The work now on the stream uses the stand-ins and the call does not wait for it.
+int leave_bounce(nbody_ctx *ctx) {
+    ctx->bounce_read = true;
+    NB_CK(ctx, cudaEventRecord(ctx->bounce_free, ctx->stream));
+    return NBODY_OK;
 }
 
 float *bounce_in(nbody_ctx *ctx, int slot, const float *from) {
@@ -518,7 +528,9 @@ int nbody_destroy(nbody_ctx *ctx) {
         cudaFree(ctx->stage);
         if (ctx->status_host) cudaFreeHost(ctx->status_host);
         else cudaFree(ctx->status);
+        if (ctx->bounce_read) cudaEventSynchronize(ctx->bounce_free);
         if (ctx->bounce) cudaFreeHost(ctx->bounce);
+        if (ctx->bounce_free) cudaEventDestroy(ctx->bounce_free);
         cudaFree(ctx->scratch.mem);
         cudaFree(ctx->vel2[1]);
         cudaFree(ctx->acc2[1]);
@@ -555,12 +567,12 @@ int nbody_upload(nbody_ctx *ctx, const float *positions4, const float *velocitie
     if (!ctx || !positions4 || !masses4) return NBODY_ERR_ARG;
     DeviceGuard dg(ctx->device);
     const size_t b4 = static_cast<size_t>(ctx->n) * sizeof(float4);
-    if (use_bounce(ctx, {positions4, velocities4, accelerations4, masses4})) {
+    const bool bounced = use_bounce(ctx, {positions4, velocities4, accelerations4, masses4});
+    if (bounced) {
         positions4 = bounce_in(ctx, 0, positions4);
         velocities4 = bounce_in(ctx, 1, velocities4);
         accelerations4 = bounce_in(ctx, 2, accelerations4);
         masses4 = bounce_in(ctx, 3, masses4);
-        ctx->bounce_read = true;
     }
     // Page-locked host buffers are read in place by one kernel; otherwise one
     // copy per array into the staging area, then the pack kernel.
@@ -582,6 +594,10 @@ int nbody_upload(nbody_ctx *ctx, const float *positions4, const float *velocitie
         else
             NB_CK(ctx, cudaMemsetAsync(ctx->acc, 0, b4, ctx->stream));
         NB_CK(ctx, nbody::pack_state(ctx->stage, ctx->stage + ctx->n, ctx->pos[0], ctx->n, ctx->stream));
+    }
+    if (bounced) {
+        const int rc = leave_bounce(ctx);
+        if (rc != NBODY_OK) return rc;
     }
     ctx->cur = 0;
     ctx->bh_pos = 0;
@@ -614,6 +630,8 @@ int nbody_download(nbody_ctx *ctx, float *positions4, float *velocities4, float 
             bounce_out(ctx, 1, velocities4);
             bounce_out(ctx, 2, accelerations4);
             bounce_out(ctx, 4, forces4);
+        } else {
+            leave_bounce(ctx);
         }
         return rc;
     }
@@ -826,6 +844,8 @@ int nbody_update_host(nbody_ctx *ctx, float *positions4, float *velocities4, flo
                 bounce_out(ctx, 1, velocities4);
                 bounce_out(ctx, 2, accelerations4);
                 bounce_out(ctx, 4, forces4);
+            } else {
+                leave_bounce(ctx);
             }
             return rc;
         }

@@ -1500,6 +1500,11 @@ int bh_walk_team(const BHWorkspace &w, int64_t n) {
     return w.walk == kWalkCell && w.bodies_per_lane == 2 ? bh_team_size(n) : 1;
 }
 
+int64_t bh_forms(const BHWorkspace &w, int64_t n, bool ensemble) {
+    const int64_t sorts = (sort_by_merging(n) ? 1 : 0) | (bh_upsweep_by_levels(n, ensemble) ? 2 : 0);
+    return ensemble ? sorts : sorts | bh_walk_team(w, n) << 2 | bh_main_sets(n) << 8;
+}
+
 bool bh_walk_writes_host(const BHWorkspace &w) { return w.walk == kWalkCell && w.bodies_per_lane == 2; }
 
 int bh_walk_form() {

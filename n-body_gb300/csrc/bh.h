@@ -103,6 +103,10 @@ cudaError_t bh_gather(int64_t n, const BHWorkspace &w, const float4 *pos_in, con
 // kernel launches it takes.
 bool bh_upsweep_by_levels(int64_t n, bool ensemble);
 int bh_upsweep_launches(int64_t n, bool ensemble);
+// The forms that a step of n bodies takes now (sort, upsweep, and of a single
+// system team size and tail), in one number: a graph captured under another is
+// not this step's. An ensemble's teams are fixed by its layout.
+int64_t bh_forms(const BHWorkspace &w, int64_t n, bool ensemble);
 cudaError_t bh_build(const float4 *pos_sorted, int64_t n, BHWorkspace &w, cudaStream_t st, int *status,
                      StageTimer *timer, const SegView &sv = SegView{});
 // The caller's arrays in the reference layout (device-mapped page-locked host

@@ -32,15 +32,14 @@ struct GraphKey {
     int64_t n = 0;
     int va = -1, key_mode = -1, integrator = -1, walk = -1, bodies_per_lane = -1;
     float dt = 0.f, eps2 = 0.f, theta2 = 0.f;
+    int64_t form[3] = {};  // bh_forms, or the direct sum's plan
     const void *host[9] = {};
     bool operator==(const GraphKey &o) const {
         if (ws != o.ws || n != o.n || va != o.va || key_mode != o.key_mode || integrator != o.integrator ||
             walk != o.walk || bodies_per_lane != o.bodies_per_lane || dt != o.dt || eps2 != o.eps2 ||
             theta2 != o.theta2)
             return false;
-        for (int i = 0; i < 9; ++i)
-            if (host[i] != o.host[i]) return false;
-        return true;
+        return std::equal(form, form + 3, o.form) && std::equal(host, host + 9, o.host);
     }
 };
 
@@ -274,6 +273,7 @@ GraphKey graph_key(const nbody_ctx *ctx) {
     k.dt = ctx->dt;
     k.eps2 = ctx->eps2;
     k.theta2 = ctx->theta2;
+    if (ctx->mode == NBODY_MODE_BH) k.form[0] = nbody::bh_forms(ctx->ws, ctx->n, false);
     k.host[8] = reinterpret_cast<const void *>(static_cast<uintptr_t>(ctx->bh_pos + 1));
     return k;
 }
@@ -813,6 +813,9 @@ bool pp_update_graphed(nbody_ctx *ctx, const float *positions4, float *velocitie
     };
     GraphKey key = graph_key(ctx);
     key.ws = ctx->scratch.mem;
+    key.form[0] = plan.sym.blocks > 0 ? plan.sym.ctas : -plan.linear_ctas;
+    key.form[1] = plan.slices;
+    key.form[2] = plan.k * 1024 + plan.threads;
     const void *arrays[9] = {mp, mv, ma, mm, mf, nullptr, nullptr, nullptr, nullptr};
     for (int i = 0; i < 9; ++i) key.host[i] = arrays[i];
     bool replayed = false;

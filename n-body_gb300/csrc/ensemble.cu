@@ -122,7 +122,7 @@ struct nbody_ensemble {
         cudaGraphExec_t exec = nullptr;
         int end_pp_cur = 0, end_bh_va = 0;
     };
-    std::map<std::tuple<int, int, int>, Graph> graphs;
+    std::map<std::tuple<int, int, int, int64_t>, Graph> graphs;  // by steps, buffers and forms
     int64_t steps_done = 0;
     nbody::EventTimer *timer = nullptr;  // non-null while profiling (steps then run without graphs)
 };
@@ -456,7 +456,7 @@ int step_once(nbody_ensemble *e) {
 }
 
 int run_graph(nbody_ensemble *e, int k) {
-    const auto key = std::make_tuple(k, e->pp_cur, e->bh_va);
+    const auto key = std::make_tuple(k, e->pp_cur, e->bh_va, e->bh_n > 0 ? nbody::bh_forms(e->ws, e->bh_n, true) : 0);
     auto it = e->graphs.find(key);
     if (it == e->graphs.end()) {
         const int pc = e->pp_cur, va = e->bh_va;

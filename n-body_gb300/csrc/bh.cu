@@ -327,12 +327,15 @@ __global__ void gather_kernel(const uint32_t *__restrict__ perm, int64_t n, cons
                               float4 *__restrict__ vel_out, float4 *__restrict__ acc_out,
                               int *__restrict__ id_out, int *status, const uint64_t *__restrict__ key_in,
                               uint64_t *__restrict__ key_out, uint32_t *__restrict__ mask,
-                              unsigned *__restrict__ broken) {
+                              unsigned *__restrict__ broken, unsigned *__restrict__ ready) {
     wait_for_launches_before();
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
     mask[i] = 0u;  // for the build that follows
-    if (i == 0) *broken = 0u;
+    if (i == 0) {
+        *broken = 0u;
+        *ready = 0u;
+    }
     uint32_t j = perm[i];
     if (j >= static_cast<uint64_t>(n)) {  // not a permutation: report, read in bounds
         record_error(status, NBODY_ERR_CAPACITY);
@@ -1028,9 +1031,13 @@ __global__ void __launch_bounds__(64, (COUNT || SEG) ? 16 : 24) cell_walk_kernel
     const float4 *__restrict__ pos, int64_t n, float eps2, float theta2, float dt, float4 *__restrict__ pos_out,
     float4 *__restrict__ vel, float4 *__restrict__ acc, float4 *__restrict__ force_out, const int *__restrict__ ids,
     unsigned long long *__restrict__ counters, float *__restrict__ phi_out, int euler, const int4 *__restrict__ work,
-    int nwork, const float4 *__restrict__ params, const uint32_t *__restrict__ P, const HostOut host, int beside) {
+    int nwork, const float4 *__restrict__ params, const uint32_t *__restrict__ P, const HostOut host, int beside,
+    unsigned *ready) {
     wait_for_launches_before();
-    if (beside & kWalkLetsNext) let_next_launch_begin();
+    if (beside & kWalkLetsNext) {  // always the first of several (bh.h)
+        if (blockIdx.x == 0 && threadIdx.x == 0) store_release(ready, 1u);
+        let_next_launch_begin();
+    }
     // One block of shared memory per warp, addressed from one base.
     struct __align__(16) WarpArea {
         int4 stk_i[kCellDepth];     // cell, mask A, mask B, box hz (float bits)
@@ -1346,6 +1353,7 @@ size_t bh_workspace_layout(int64_t n, void *base, BHWorkspace *w) {
     w->bbox_partial = static_cast<float *>(take(sizeof(float) * 6 * kBBoxBlocks));
     w->bbox_counter = static_cast<unsigned *>(take(sizeof(unsigned) * 4));
     w->broken = static_cast<unsigned *>(take(sizeof(unsigned)));
+    w->ready = static_cast<unsigned *>(take(sizeof(unsigned)));
     w->tree.lo = static_cast<int *>(take(sizeof(int) * nn));
     w->tree.hi = static_cast<int *>(take(sizeof(int) * nn));
     w->tree.delta = static_cast<int *>(take(sizeof(int) * nn));
@@ -1408,7 +1416,8 @@ cudaError_t bh_gather(int64_t n, const BHWorkspace &w, const float4 *pos_in, con
                       int *id_out, cudaStream_t st, int *status, StageTimer *timer) {
     if (timer) timer->begin(kStageGather, st);
     launch_behind(gather_kernel, dim3(grid_for(n, 256)), dim3(256), 0, st, w.vals[0], n, pos_in, vel_in, acc_in,
-                  id_in, pos_out, vel_out, acc_out, id_out, status, nullptr, nullptr, w.mask, w.broken);
+                  id_in, pos_out, vel_out, acc_out, id_out, status, nullptr, nullptr, w.mask, w.broken,
+                  w.ready);
     if (timer) timer->end(kStageGather, st);
     return cudaGetLastError();
 }
@@ -1480,14 +1489,14 @@ void launch_walk(const BHWorkspace &w, unsigned blocks, cudaStream_t st, const u
         if (w.walk == kWalkCell && host.pos) {
             launch_behind(cell_walk_kernel<COUNT, POT, SEG, GUARD, true>, dim3(blocks * 4), dim3(64), 0, st, w.nodes,
                           w.kids, node_total, pos, n, eps2, theta2, dt, pos_out, vel, acc, force_out, ids, counters,
-                          phi_out, euler, work, nwork, params, P, host, beside);
+                          phi_out, euler, work, nwork, params, P, host, beside, w.ready);
             return;
         }
     }
     if (w.walk == kWalkCell)
         launch_behind(cell_walk_kernel<COUNT, POT, SEG, GUARD>, dim3(blocks * 4), dim3(64), 0, st, w.nodes, w.kids,
                       node_total, pos, n, eps2, theta2, dt, pos_out, vel, acc, force_out, ids, counters, phi_out,
-                      euler, work, nwork, params, P, host, beside);
+                      euler, work, nwork, params, P, host, beside, w.ready);
     else
         traverse2_kernel<COUNT, POT, SEG, GUARD><<<blocks, 256, 0, st>>>(w.nodes, node_total, pos, n, eps2, theta2,
                                                                          dt, pos_out, vel, acc, force_out, ids,
@@ -1541,6 +1550,7 @@ cudaError_t bh_traverse(const float4 *pos_sorted, int64_t n, const BHWorkspace &
         a.euler = euler;
         a.host = host;
         a.beside = beside;
+        a.ready = w.ready;
         cudaError_t e = cudaSuccess;
         const unsigned blocks = static_cast<unsigned>((main * 32 + 255) / 256);
         if (team > 1)
@@ -1625,7 +1635,8 @@ cudaError_t bh_ensemble_step(int64_t n, BHWorkspace &w, const BHEnsembleTables &
     // Sorted keys into keys[0] (the build reads them there), permutation in vals[0].
     uint64_t *ksorted = w.keys[0];
     launch_behind(gather_kernel, dim3(grid_for(n, 256)), dim3(256), 0, st, v0, n, P, V, A, I, Po, Vo, Ao, Io, status,
-                  e.keys_orig, ksorted, w.mask, w.broken);
+                  e.keys_orig, ksorted, w.mask, w.broken,
+                  w.ready);
     if (tm) tm->end(kStageGather, st);
     err = cudaGetLastError();
     if (err != cudaSuccess) return err;
@@ -1659,6 +1670,7 @@ cudaError_t bh_ensemble_step(int64_t n, BHWorkspace &w, const BHEnsembleTables &
             a.params = e.params;
             a.P = w.P;
             a.beside = beside;
+        a.ready = w.ready;
             err = bh_team_walk(a, team, !e.all_soft, sets, st);
             if (err != cudaSuccess) return err;
         } else {

@@ -70,7 +70,10 @@ struct BHWorkspace {
     uint32_t *mask = nullptr;
     uint32_t *P = nullptr;  // n + 1 entries; P[n] = record count
     unsigned long long *scan_words = nullptr;
-    unsigned *broken = nullptr;  // raised by a build whose keys or prefix sums are not whole; cleared by the gather
+    // Two words that the gather clears: raised by a build whose keys or prefix
+    // sums are not whole, and by the first of several walks once it has waited.
+    unsigned *broken = nullptr;
+    unsigned *ready = nullptr;
     BHNode *nodes = nullptr;  // up to 2n records
     int *kids = nullptr;      // child table: 8 places per cell record, by key digit; -1: no child
     // Traversal counters (pairwise evaluations, warp record visits): the
@@ -147,11 +150,18 @@ struct TeamWalk {
     HostOut host;
     int64_t first = 0;  // the system's first set
     int beside = 0;     // kWalkLetsNext, kWalkWaitsLast
+    unsigned *ready = nullptr;
 };
 // Walks of one step side by side: launches that write different bodies and read
 // what no walk writes. Each but the last lets the next begin when its own last
-// CTAs have; each but the first begins without a wait and ends after the one
-// before (so that what follows the last follows all).
+// CTAs have; each but the first begins without a wait for the one before it and
+// ends after it (so that what follows the last follows all). A launch that has
+// begun that way has not waited for the build, and the wait is what makes the
+// build's writes visible: the first walk, which has waited, stores *ready with a
+// release before it lets the next begin, and the others' first threads load it
+// with an acquire, which with the block's barrier orders the block's reads behind
+// the build. The gather in front of the build clears the word; a block that does
+// not find it set waits for the launch before it to end.
 constexpr int kWalkLetsNext = 1, kWalkWaitsLast = 2;
 // Warps per set of a system of n bodies: 1 is cell_walk_kernel.
 int bh_team_size(int64_t n);

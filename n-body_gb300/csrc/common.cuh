@@ -106,6 +106,15 @@ __device__ __forceinline__ void wait_for_launches_before() { asm volatile("gridd
 // come here or ended, instead of when all have ended.
 __device__ __forceinline__ void let_next_launch_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+__device__ __forceinline__ void store_release(unsigned *p, unsigned v) {
+    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ unsigned load_acquire(const unsigned *p) {
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
 // 1/sqrt(x), hardware approximation, flush-to-zero (inputs here are >= eps^2).
 __device__ __forceinline__ float rsqrt_ftz(float x) {
     float y;

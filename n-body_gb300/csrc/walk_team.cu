@@ -113,11 +113,18 @@ __global__ void __launch_bounds__(32 * W, W >= 16 && !SEG ? 1 : 32 / W) team_wal
     const float4 *__restrict__ pos, int64_t n, float eps2, float theta2, float dt, float4 *__restrict__ pos_out,
     float4 *__restrict__ vel, float4 *__restrict__ acc, float4 *__restrict__ force_out, const int *__restrict__ ids,
     unsigned long long *__restrict__ counters, int euler, const int4 *__restrict__ work,
-    const float4 *__restrict__ params, const uint32_t *__restrict__ P, const HostOut host, int64_t first, int beside) {
+    const float4 *__restrict__ params, const uint32_t *__restrict__ P, const HostOut host, int64_t first, int beside,
+    unsigned *ready) {
     __shared__ __align__(16) TeamArea<W> A;
     constexpr int S = TeamArea<W>::S;
-    if (!(beside & kWalkWaitsLast)) wait_for_launches_before();
-    if (beside & kWalkLetsNext) let_next_launch_begin();
+    // Beside the walk before it (bh.h): what the build wrote is seen through that
+    // walk's word, or, where it cannot be seen yet, by waiting for its end.
+    if (!(beside & kWalkWaitsLast) || !__syncthreads_or(threadIdx.x == 0 && load_acquire(ready) != 0u))
+        wait_for_launches_before();
+    if (beside & kWalkLetsNext) {
+        if (!(beside & kWalkWaitsLast) && blockIdx.x == 0 && threadIdx.x == 0) store_release(ready, 1u);
+        let_next_launch_begin();
+    }
     unsigned long long n_pairs = 0, n_visits = 0;
     float phi = 0.f;  // no potential in this form
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -357,7 +364,7 @@ cudaError_t launch_form(const TeamWalk &a, unsigned sets, cudaStream_t st) {
     const auto launch = [&](auto kernel) {
         return launch_behind(kernel, dim3(sets), dim3(32 * W), 0, st, a.nodes, a.kids, a.node_total, a.pos, a.n, a.eps2,
                              a.theta2, a.dt, a.pos_out, a.vel, a.acc, a.force_out, a.ids, a.counters, a.euler, a.work,
-                             a.params, a.P, a.host, a.first, a.beside);
+                             a.params, a.P, a.host, a.first, a.beside, a.ready);
     };
     if constexpr (!SEG)
         if (a.host.pos) return launch(team_walk_kernel<W, COUNT, SEG, GUARD, true>);

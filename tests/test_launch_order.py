@@ -72,6 +72,16 @@ def test_kernel_waits_before_it_touches_memory(name):
     assert WAIT in body, f"{name} is launched behind the kernel before it and never waits for it"
     before = body[:body.index(WAIT)]
     touched = [p for p in pointers if re.search(rf"\b{p}\b", before)]
-    assert not touched, f"{name} uses {touched} before it waits"
-    if "beside" not in before:  # a walk beside another waits where it ends
+    if "kWalkWaitsLast" in before:  # begins beside the walk before it, by that walk's word
+        assert "load_acquire(ready)" in before, f"{name} skips the wait without an acquire of what it reads"
+        touched.remove("ready")
+    else:
         assert body.count(WAIT) == 1
+    assert not touched, f"{name} uses {touched} before it waits"
+
+
+@pytest.mark.parametrize("name", ["cell_walk_kernel", "team_walk_kernel"])
+def test_walk_says_that_it_has_waited_before_it_lets_the_next_begin(name):
+    body = KERNELS[name][1]
+    said, let = body.index("store_release(ready"), body.index("let_next_launch_begin();")
+    assert body.index(WAIT) < said < let

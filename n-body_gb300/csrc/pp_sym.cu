@@ -38,7 +38,6 @@
 // 2^40, softening below 2^-80 or beyond 2^83), one more operation per pair keeps
 // pp.cu's order (m * inv) * inv^2.
 #include <algorithm>
-#include <vector>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -411,7 +410,7 @@ SymPlan pp_sym_plan(int64_t n, int sms) {
     // else one even cut over all blocks.
     const int total = sym_weight(p, p.blocks);
     auto weight_of = [&](int b) { return sym_weight(p, b + 1) - sym_weight(p, b); };
-    std::vector<int> of(static_cast<size_t>(p.blocks));
+    int of[kSymMaxBlocks];
     int given = 0, longest = 0;
     for (int b = 0; b < p.blocks; ++b)
         given += of[b] = static_cast<int>(static_cast<int64_t>(weight_of(b)) * p.ctas / total);

@@ -430,7 +430,8 @@ def bench_bh(args, world, rank, local, dist):
         stages[name] = st
     roofline = {"bound": "fp32", "achieved": round(achieved, 3), "peak": round(fp32, 3), "unit": "TFLOP/s",
                 "frac": round(achieved / fp32, 4), "traffic": profile_traffic("bh_traverse"),
-                "kernel": "traverse2_kernel" if os.environ.get("NBODY_BH_WALK") == "union" else "cell_walk_kernel",
+                "kernel": "traverse2_kernel" if os.environ.get("NBODY_BH_WALK") == "union"
+                else "cell_walk_kernel + team_walk_kernel",
                 "kernel_ms_per_launch": round(t_launch * 1e3, 4),
                 "work": {"pair_evaluations_per_step": pairs, "per_body": round(pairs / n, 1),
                          "warp_record_visits_per_step": visits,

@@ -427,8 +427,9 @@ __global__ void radix_tree_kernel(const uint64_t *__restrict__ k, int64_t n, Bin
 // P[n] = the number of records: one pass. A CTA takes the next tile (so that
 // every tile it waits on is already running), publishes its tile's count, adds
 // up the tiles before it 32 at a time until one that already knows its prefix
-// (bounded waits), and publishes its own prefix. words: [0] the tile counter,
-// then a word per tile, all zero before. As a count kernel and a three-kernel
+// (bounded waits), and publishes its own prefix (decoupled look-back: Merrill,
+// Garland, "Single-pass Parallel Prefix Scan with Decoupled Look-back", 2016).
+// words: [0] the tile counter, then a word per tile, all zero before. As a count kernel and a three-kernel
 // scan this took 13 us and three launch gaps for any small n.
 constexpr int kScanThreads = 512;
 constexpr int kScanItems = 4;

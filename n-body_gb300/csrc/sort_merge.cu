@@ -11,7 +11,7 @@
 // two at a time above, every CTA producing 2,048 pairs from the part of two runs
 // that a search along the merge path gives it (merge_pass_kernel). Taking the
 // left run first where keys are equal keeps the sort stable, so the permutation
-// is the radix sort's. GB300, us, radix / merge: 4,096 pairs 105 / 17, 30,001
+// is the radix sort's. (Merge path: Green, McColl, Bader, "GPU Merge Path", ICS 2012.) GB300, us, radix / merge: 4,096 pairs 105 / 17, 30,001
 // 120 / 22, 65,536 121 / 26, 262,144 137 / 53, 2^20 212 / 121, 2^22 553 / 452.
 // A tile of 2,048 pairs takes 10 us, a pass by searching 5 us up to 2^17 pairs, a
 // merge pass 7 us while its launch and the chain of its searches bound it and

@@ -103,7 +103,7 @@ __device__ __forceinline__ void add_kids(const float4 *xy, const float4 *zm, int
     for (; j < cnt; ++j) add_kid<COUNT, GUARD, ALL>(xy[j], zm[j], useA, useB, nx, ny, nz, e2, fx, fy, fz, n_pairs);
 }
 
-// Registers: 64 (32 warps per SM), and up to 94 for the largest team of a
+// Registers: 64 (32 warps per SM), and up to 98 for the largest team of a
 // single system, which rarely has more than one CTA per SM anyway (4,096
 // bodies: 57 against 64 us at 64 registers); 48 registers lose at every size
 // (65,536 bodies, 4 warps: 405 against 302 us).
@@ -396,6 +396,10 @@ cudaError_t launch_team(const TeamWalk &a, bool guard, unsigned sets, cudaStream
 // 11.7, 60 of 65,536: 1 warp 11.2, 4 warps 11.7): 4 from 32,768 on although 8 is
 // level with it for one system up to 2^17, and 16 only below the sizes at which
 // ensembles turn to Barnes-Hut.
+// What that costs an ensemble that fills the chip: steps of 2,048 ragged systems of
+// 256 to 131,072 bodies 140.0 ms by this rule, 138.1 by teams of 4 throughout, 130.8
+// by one warp per set; what it buys a lone system stands in the table (one warp per
+// set takes 5 to 7 times as long up to 30,001 bodies).
 constexpr int64_t kMaxTeams = 458752;  // with the tails below: 393,216 bodies 1.357 by fours, 1.381 ms by one warp
 int bh_team_size(int64_t n) {
     if (const char *e = std::getenv("NBODY_BH_TEAM")) {  // 1, 2, 4, 8 or 16: that team for every size

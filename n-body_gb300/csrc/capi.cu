@@ -367,6 +367,15 @@ bool pageable(std::initializer_list<const void *> arrays, size_t bytes) {
     return true;
 }
 
+// While it lives, this thread may allocate and wait for events although some
+// stream is being captured by a caller who forbids both to everyone: neither
+// touches that stream, and refused they would end its capture.
+struct CaptureAside {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    CaptureAside() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~CaptureAside() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // Whether a call on these arrays takes the stand-ins (made, and free to be
 // written, when it does).
 bool use_bounce(nbody_ctx *ctx, std::initializer_list<const void *> arrays) {
@@ -376,6 +385,7 @@ bool use_bounce(nbody_ctx *ctx, std::initializer_list<const void *> arrays) {
     if (cudaStreamIsCapturing(ctx->stream, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) return false;
     const size_t b4 = static_cast<size_t>(ctx->n) * sizeof(float4);
     if (!pageable(arrays, b4)) return false;
+    const CaptureAside aside;
     if (!ctx->bounce) {
         if (!ctx->bounce_free && cudaEventCreateWithFlags(&ctx->bounce_free, cudaEventDisableTiming) != cudaSuccess)
             ctx->bounce_free = nullptr;

@@ -138,19 +138,20 @@ nbody::PPPlan plan_of(const nbody_ctx *ctx, int64_t n) {
     return nbody::pp_scratch_plan(ctx->scratch, [&](bool sym) { return nbody::pp_plan(n, ctx->device, true, sym); });
 }
 
+struct DeviceMemory {
+    cudaStream_t stream;
+    cudaError_t alloc(void **p, size_t bytes) {
+        const cudaError_t e = cudaMalloc(p, bytes);
+        if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+        return e;
+    }
+    cudaError_t clear(void *p, size_t bytes) { return cudaMemsetAsync(p, 0, bytes, stream); }
+    cudaError_t wait() { return cudaStreamSynchronize(stream); }
+    void free(void *p) { cudaFree(p); }
+};
+
 int ensure_scratch(nbody_ctx *ctx, int64_t n, nbody::PPPlan &plan) {
-    struct {
-        cudaStream_t stream;
-        cudaError_t alloc(void **p, size_t bytes) {
-            const cudaError_t e = cudaMalloc(p, bytes);
-            if (e == cudaErrorMemoryAllocation) cudaGetLastError();
-            return e;
-        }
-        cudaError_t clear(void *p, size_t bytes) { return cudaMemsetAsync(p, 0, bytes, stream); }
-        cudaError_t wait() { return cudaStreamSynchronize(stream); }
-        void free(void *p) { cudaFree(p); }
-    } device{ctx->stream};
-    NB_CK(ctx, nbody::pp_scratch_ensure(ctx->scratch, plan, device,
+    NB_CK(ctx, nbody::pp_scratch_ensure(ctx->scratch, plan, DeviceMemory{ctx->stream},
                                         [&](bool sym) { return nbody::pp_plan(n, ctx->device, true, sym); }));
     return NBODY_OK;
 }
@@ -169,6 +170,8 @@ int read_status(nbody_ctx *ctx) {
     if (h != NBODY_OK && ctx->scratch.mem) {
         // A kernel gave up part-way: its arrival counters may be left non-zero.
         NB_CK(ctx, cudaMemsetAsync(ctx->scratch.mem, 0, ctx->scratch.bytes, ctx->stream));
+        if (ctx->scratch.first != ctx->scratch.mem)
+            NB_CK(ctx, cudaMemsetAsync(ctx->scratch.first, 0, nbody::kFirstScratch, ctx->stream));
         NB_CK(ctx, cudaStreamSynchronize(ctx->stream));
     }
     return h;
@@ -514,6 +517,10 @@ int nbody_create(nbody_ctx **out, int device, int mode, int64_t n, float dt, flo
     }
     if (rc == NBODY_OK && mode == NBODY_MODE_BH) rc = ensure_workspace(ctx, n);
     if (rc == NBODY_OK) {
+        const cudaError_t e = nbody::pp_scratch_first(ctx->scratch, DeviceMemory{ctx->stream});
+        if (e != cudaSuccess) rc = fail(ctx, e);
+    }
+    if (rc == NBODY_OK) {
         cudaError_t e = ctx->status_host ? cudaSuccess : cudaMemsetAsync(ctx->status, 0, sizeof(int), ctx->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess) rc = fail(ctx, e);
@@ -541,7 +548,8 @@ int nbody_destroy(nbody_ctx *ctx) {
         if (ctx->bounce_read) cudaEventSynchronize(ctx->bounce_free);
         if (ctx->bounce) cudaFreeHost(ctx->bounce);
         if (ctx->bounce_free) cudaEventDestroy(ctx->bounce_free);
-        cudaFree(ctx->scratch.mem);
+        if (ctx->scratch.mem != ctx->scratch.first) cudaFree(ctx->scratch.mem);
+        cudaFree(ctx->scratch.first);
         cudaFree(ctx->vel2[1]);
         cudaFree(ctx->acc2[1]);
         cudaFree(ctx->ids[0]);

@@ -15,12 +15,32 @@ namespace nbody {
 // for 8M bodies.
 constexpr size_t kArrivalsArea = 64 << 10;
 
+// Scratch that a context has from the start: enough for the plans of up to 510
+// bodies (eight slices of 16 bytes a body). They took one slice and no scratch
+// before short slices came (pp_small_shape), so that their first call may itself
+// be one that the caller captures, where nothing can be allocated. It is kept
+// beside a larger one (giving it back would cost the first larger call a wait and
+// a free, 12 us).
+constexpr size_t kFirstScratch = kArrivalsArea + 510 * 8 * 16;
+
 struct PPScratch {
     void *mem = nullptr;
     size_t bytes = 0;
     size_t arrivals = 0;         // bytes of arrival counters of the plan that used it last
     size_t refused = SIZE_MAX;   // a pair-once plan of this many bytes could not be had
+    void *first = nullptr;       // kFirstScratch bytes, once pp_scratch_first has been called
 };
+
+// The context's first scratch.
+template <class Mem>
+cudaError_t pp_scratch_first(PPScratch &s, Mem &&m) {
+    cudaError_t e = m.alloc(&s.first, kFirstScratch);
+    if (e != cudaSuccess) return e;
+    s.mem = s.first;
+    s.bytes = kFirstScratch;
+    s.arrivals = kArrivalsArea;
+    return m.clear(s.first, kFirstScratch);
+}
 
 inline void pp_scratch_reserve(PPPlan &plan) {
     if (plan.partial_bytes == 0 || plan.arrivals_bytes >= kArrivalsArea) return;
@@ -59,22 +79,23 @@ cudaError_t pp_scratch_ensure(PPScratch &s, PPPlan &plan, Mem &&m, PlanOf &&plan
             plan = pp_scratch_plan(s, plan_of);
             e = plan.partial_bytes > s.bytes ? m.alloc(&more, plan.partial_bytes) : cudaSuccess;
         }
-        if (e == cudaErrorMemoryAllocation && s.mem) {
+        if (e == cudaErrorMemoryAllocation && s.mem != s.first) {
             if (const cudaError_t w = m.wait()) return w;
             m.free(s.mem);
-            s.mem = nullptr;
-            s.bytes = 0;
+            s.mem = s.first;
+            s.bytes = s.first ? kFirstScratch : 0;
+            s.arrivals = s.first ? kArrivalsArea : 0;
             e = m.alloc(&more, plan.partial_bytes);
         }
         if (e != cudaSuccess) return e;
         if (more) {
             e = m.clear(more, plan.partial_bytes);
-            if (e == cudaSuccess && s.mem) e = m.wait();
+            if (e == cudaSuccess && s.mem != s.first) e = m.wait();
             if (e != cudaSuccess) {
                 m.free(more);
                 return e;
             }
-            if (s.mem) m.free(s.mem);
+            if (s.mem != s.first) m.free(s.mem);
             s.mem = more;
             s.bytes = plan.partial_bytes;
             s.arrivals = plan.arrivals_bytes;

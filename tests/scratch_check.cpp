@@ -130,9 +130,32 @@ void counters() {
     CHECK(c.call(1) == cudaSuccess && c.d.clears == clears + 2);
 }
 
+void first_scratch() {
+    Context c;
+    c.d.budget = 25 * kMB;
+    CHECK(pp_scratch_first(c.s, c.d) == cudaSuccess && c.s.mem == c.s.first && c.d.clears == 1);
+    const auto small = [](bool) {
+        PPPlan p;
+        p.arrivals_bytes = 256;
+        p.partial_bytes = 256 + 510 * 8 * 16;
+        return p;
+    };
+    const int calls = c.d.calls();
+    PPPlan p = pp_scratch_plan(c.s, small);
+    CHECK(pp_scratch_ensure(c.s, p, c.d, small) == cudaSuccess && c.d.calls() == calls && c.s.mem == c.s.first);
+    // A larger one beside it: no wait, nothing given back, then or when that one makes room.
+    CHECK(c.call(1) == cudaSuccess && c.s.mem != c.s.first && c.d.waits == 0 && c.d.frees == 0);
+    CHECK(c.call(18) == cudaSuccess && c.d.waits == 1 && c.d.frees == 1 && c.d.live.count(c.s.first) == 1);
+    CHECK(c.call(60) == cudaErrorMemoryAllocation && c.s.mem == c.s.first && c.s.bytes == kFirstScratch);
+    CHECK(c.d.used == kFirstScratch);
+    p = pp_scratch_plan(c.s, small);
+    CHECK(pp_scratch_ensure(c.s, p, c.d, small) == cudaSuccess && c.s.mem == c.s.first);
+}
+
 }  // namespace
 
 int main() {
+    first_scratch();
     plenty();
     pair_once_refused();
     ordered_refused();

@@ -7,6 +7,7 @@
 // memory its kernels need, and a non-blocking stream (replaceable with
 // nbody_set_stream).
 #include <cuda_runtime.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <cstdlib>
@@ -32,7 +33,7 @@ struct GraphKey {
     int64_t n = 0;
     int va = -1, key_mode = -1, integrator = -1, walk = -1, bodies_per_lane = -1;
     float dt = 0.f, eps2 = 0.f, theta2 = 0.f;
-    int64_t form[3] = {};  // bh_forms, or the direct sum's plan
+    int64_t form[3] = {};  // bh_forms where a switch is set, or the direct sum's plan
     const void *host[9] = {};
     bool operator==(const GraphKey &o) const {
         if (ws != o.ws || n != o.n || va != o.va || key_mode != o.key_mode || integrator != o.integrator ||
@@ -264,6 +265,14 @@ int bh_step(nbody_ctx *ctx, cudaEvent_t join = nullptr, const float4 *masses4 = 
     return NBODY_OK;
 }
 
+// Whether a variable of the library's is set at all: one pass over the
+// environment instead of one for each of them.
+bool any_switch() {
+    for (char **e = environ; e && *e; ++e)
+        if (std::strncmp(*e, "NBODY_", 6) == 0) return true;
+    return false;
+}
+
 GraphKey graph_key(const nbody_ctx *ctx) {
     GraphKey k;
     k.ws = ctx->ws_mem;
@@ -276,7 +285,8 @@ GraphKey graph_key(const nbody_ctx *ctx) {
     k.dt = ctx->dt;
     k.eps2 = ctx->eps2;
     k.theta2 = ctx->theta2;
-    if (ctx->mode == NBODY_MODE_BH) k.form[0] = nbody::bh_forms(ctx->ws, ctx->n, false);
+    // Without a switch the forms follow from n (0).
+    if (ctx->mode == NBODY_MODE_BH && any_switch()) k.form[0] = 1 + nbody::bh_forms(ctx->ws, ctx->n, false);
     k.host[8] = reinterpret_cast<const void *>(static_cast<uintptr_t>(ctx->bh_pos + 1));
     return k;
 }
@@ -388,8 +398,8 @@ bool use_bounce(nbody_ctx *ctx, std::initializer_list<const void *> arrays) {
     if (cudaStreamIsCapturing(ctx->stream, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) return false;
     const size_t b4 = static_cast<size_t>(ctx->n) * sizeof(float4);
     if (!pageable(arrays, b4)) return false;
-    const CaptureAside aside;
     if (!ctx->bounce) {
+        const CaptureAside aside;
         if (!ctx->bounce_free && cudaEventCreateWithFlags(&ctx->bounce_free, cudaEventDisableTiming) != cudaSuccess)
             ctx->bounce_free = nullptr;
         if (!ctx->bounce_free ||
@@ -400,8 +410,11 @@ bool use_bounce(nbody_ctx *ctx, std::initializer_list<const void *> arrays) {
             return false;
         }
     }
-    if (ctx->bounce_read && cudaEventSynchronize(ctx->bounce_free) != cudaSuccess) return false;
-    ctx->bounce_read = false;
+    if (ctx->bounce_read) {
+        const CaptureAside aside;
+        if (cudaEventSynchronize(ctx->bounce_free) != cudaSuccess) return false;
+        ctx->bounce_read = false;
+    }
     return true;
 }
 

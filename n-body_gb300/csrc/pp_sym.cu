@@ -332,7 +332,8 @@ __global__ void __launch_bounds__(kSymT) pp_sym_sum_kernel(const float4 *__restr
     wait_for_launches_before();
     const int to = blockIdx.x / (kSymB / kSymT), i0 = (blockIdx.x % (kSymB / kSymT)) * kSymT + threadIdx.x;
     const int64_t i = static_cast<int64_t>(to) * kSymB + i0;
-    if (i >= n) return;
+    // One thread's load for the block: every warp's took 0.3 us of a step.
+    const bool gave_up = threadIdx.x == 0 && parts[-1] != 0.f;
     const int first = sym_first(p, to), past = sym_first(p, to + 1);
     int lo = 0, hi = p.ctas;  // the range of the block's first tile: begin[lo] <= first < begin[hi]
     while (hi - lo > 1) {
@@ -382,7 +383,7 @@ __global__ void __launch_bounds__(kSymT) pp_sym_sum_kernel(const float4 *__restr
             fz += vz[u];
         }
     }
-    if (parts[-1] != 0.f) return;
+    if (__syncthreads_or(gave_up) || i >= n) return;
     if (g.pos_out) integrate_body(i, pos[i], fx, fy, fz, g);
     else if (g.force) g.force[i] = make_float4(fx, fy, fz, 0.f);
 }
